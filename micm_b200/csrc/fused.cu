@@ -269,103 +269,49 @@ namespace micmb
     return w;
   }
 
-  void SolveFused(micmb_solver& s, micmb_state& st, double dt, micmb_solver_stats* stats, int32_t* per_cell_status,
-                  int32_t* per_cell_accepted, const FusedArgs* adj)
+  namespace
   {
-    const auto& m = *s.mech;
-    micmb_fused_config cfg = s.fused;
-    if (cfg.lu_in_shared && FusedWarpsPerCta(s, cfg) < 1)
-      cfg.lu_in_shared = 0;
-    const int warps = FusedWarpsPerCta(s, cfg);
-    if (warps < 1)
-      throw Error(MICMB_ERR_UNSUPPORTED, "mechanism too large for the fused kernel's shared-memory working set");
-    if (!s.dev.has_warp)
-      throw Error(MICMB_ERR_UNSUPPORTED, "mechanism exceeds the fused kernel's 16-bit table positions (nnz <= 65534)");
-    const bool lu_shared = cfg.lu_in_shared != 0;
-    WarpLayout W = MakeLayout(m.S, m.R, s.params.stages, (int32_t)m.info_rxn.size(), m.nnz, lu_shared);
-    const size_t smem = (size_t)W.per_warp * sizeof(double) * warps;
-    const int threads = warps * kWarp;
-    auto kernel = lu_shared ? k_fused<true> : k_fused<false>;
-    MICMB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int per_sm = 0;
-    MICMB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
-    if (per_sm < 1)
-      throw Error(MICMB_ERR_UNSUPPORTED, "fused kernel cannot be resident with this configuration");
-    if (cfg.ctas_per_sm > 0)
-      per_sm = std::min(per_sm, cfg.ctas_per_sm);
-    int64_t grid = (int64_t)per_sm * s.sm_count;
-    // an adjoint chunk brings its own cell range (n_cells > 0, pointers already offset)
-    const int64_t n = (adj && adj->n_cells > 0)
-                          ? adj->n_cells
-                          : (st.solve_limit > 0 ? std::min<int64_t>(st.solve_limit, st.n_cells) : st.n_cells);
-    grid = std::max<int64_t>(1, std::min<int64_t>(grid, (n + warps - 1) / warps));
-
-    FusedArgs A{};
-    if (adj)
-      A = *adj;
-    A.n_cells = n;
-    A.L = st.L;
-    if (!adj)
+    // arguments of a per-cell solve of n cells, and the counters it starts from
+    FusedArgs PerCellArgs(micmb_state& st, const FusedArgs* adj, int64_t n)
     {
-      A.variables_in = st.variables.as<double>();
-      A.variables_out = st.variables.as<double>();
-    }
-    if (!A.rate_constants)
-      A.rate_constants = st.rate_constants.as<double>();
-    A.keq = st.keq.as<double>();
-    A.atol = st.atol.as<double>();
-    A.rtol = st.rtol;
-    char* cbase = st.counters.as<char>();
-    A.next_cell = reinterpret_cast<int32_t*>(cbase + 8);
-    A.stats = reinterpret_cast<unsigned long long*>(cbase + 64);
-    // per-cell outputs cover the whole state, whatever prefix this call solves
-    if (!st.status.p)
-      st.status = DeviceMemory(sizeof(int32_t) * std::max<int64_t>(st.n_cells, 1));
-    if (!st.accepted.p)
-      st.accepted = DeviceMemory(sizeof(int32_t) * std::max<int64_t>(st.n_cells, 1));
-    if (!A.cell_status)
-      A.cell_status = st.status.as<int32_t>();
-    if (!A.cell_accepted)
-      A.cell_accepted = st.accepted.as<int32_t>();
-    if (!lu_shared)
-    {
-      const int64_t slots = grid * warps;
-      const int64_t stride = ((int64_t)m.nnz + 1 + 31) & ~31ll;
-      if (st.lu_slot_count < slots * stride || !st.lu_slots.p)
-      {
-        st.lu_slots = DeviceMemory(sizeof(double) * (size_t)(slots * stride));
-        st.lu_slot_count = slots * stride;
-      }
-      A.lu_global = st.lu_slots.as<double>();
-      A.lu_slot_stride = stride;
-    }
-    MICMB_CUDA(cudaMemsetAsync(cbase, 0, 160, st.stream));
-    if (n > 0 && !m.constraints.empty())
-    {
-      // algebraic constraints: the one-cell-per-thread kernel is the fused form that has them
+      FusedArgs A{};
       if (adj)
-        throw Error(MICMB_ERR_UNSUPPORTED, "the adjoint does not cover algebraic constraints");
-      if (!SolveFusedThread(s, st, A, dt))
-        throw Error(MICMB_ERR_UNSUPPORTED, "one-cell-per-thread kernel cannot be resident");
-    }
-    else if (n > 0)
-    {
-      bool done = false;
-      if (s.fused.variant == 0)
-        done = SolveFusedStream(s, st, dt, A);
-      else if (s.fused.variant == 2)
-        done = SolveFusedThread(s, st, A, dt);
-      if (!done)
+        A = *adj;
+      A.n_cells = n;
+      A.L = st.L;
+      if (!adj)
       {
-        if (A.ckpt_k)
-          throw Error(MICMB_ERR_INTERNAL, "the direct fused kernel stores no stage vectors");
-        const StepBounds B = step_bounds(s.params, dt);
-        kernel<<<(unsigned)grid, threads, smem, st.stream>>>(s.dev, s.params, B, A, W);
-        MICMB_CUDA(cudaGetLastError());
+        A.variables_in = st.variables.as<double>();
+        A.variables_out = st.variables.as<double>();
       }
+      if (!A.rate_constants)
+        A.rate_constants = st.rate_constants.as<double>();
+      A.keq = st.keq.as<double>();
+      A.atol = st.atol.as<double>();
+      A.rtol = st.rtol;
+      char* cbase = st.counters.as<char>();
+      A.next_cell = reinterpret_cast<int32_t*>(cbase + 8);
+      A.stats = reinterpret_cast<unsigned long long*>(cbase + 64);
+      // per-cell outputs cover the whole state, whatever prefix this call solves
+      if (!st.status.p)
+        st.status = DeviceMemory(sizeof(int32_t) * std::max<int64_t>(st.n_cells, 1));
+      if (!st.accepted.p)
+        st.accepted = DeviceMemory(sizeof(int32_t) * std::max<int64_t>(st.n_cells, 1));
+      if (!A.cell_status)
+        A.cell_status = st.status.as<int32_t>();
+      if (!A.cell_accepted)
+        A.cell_accepted = st.accepted.as<int32_t>();
+      MICMB_CUDA(cudaMemsetAsync(cbase, 0, 160, st.stream));
+      return A;
     }
-    if (stats || per_cell_status || per_cell_accepted)
+
+    // waits for a per-cell solve and brings back what the caller asked for
+    void ReadPerCellResults(micmb_state& st, const FusedArgs& A, double dt, micmb_solver_stats* stats,
+                            int32_t* per_cell_status, int32_t* per_cell_accepted)
     {
+      if (!stats && !per_cell_status && !per_cell_accepted)
+        return;
+      const int64_t n = A.n_cells;
       unsigned long long hs[9];
       MICMB_CUDA(cudaMemcpyAsync(hs, A.stats, sizeof(hs), cudaMemcpyDeviceToHost, st.stream));
       if (per_cell_status)
@@ -376,7 +322,7 @@ namespace micmb
                                    st.stream));
       MICMB_CUDA(cudaStreamSynchronize(st.stream));
       int32_t err_flag = 0;
-      MICMB_CUDA(cudaMemcpy(&err_flag, cbase + 16, sizeof(int32_t), cudaMemcpyDeviceToHost));
+      MICMB_CUDA(cudaMemcpy(&err_flag, st.counters.as<char>() + 16, sizeof(int32_t), cudaMemcpyDeviceToHost));
       if (err_flag)
         throw Error(MICMB_ERR_TIMEOUT, "fused kernel: a pipeline wait timed out");
       if (stats)
@@ -405,5 +351,94 @@ namespace micmb
         }
       }
     }
+  }  // namespace
+
+  void SolveFused(micmb_solver& s, micmb_state& st, double dt, micmb_solver_stats* stats, int32_t* per_cell_status,
+                  int32_t* per_cell_accepted, const FusedArgs* adj)
+  {
+    const auto& m = *s.mech;
+    // an adjoint chunk brings its own cell range (n_cells > 0, pointers already offset)
+    const int64_t n = (adj && adj->n_cells > 0)
+                          ? adj->n_cells
+                          : (st.solve_limit > 0 ? std::min<int64_t>(st.solve_limit, st.n_cells) : st.n_cells);
+    if (n > 0 && s.fused.variant == 0 && GroupVariantApplies(s, n))
+    {
+      const FusedArgs A = PerCellArgs(st, adj, n);
+      SolveFusedGroup(s, st, A, dt);
+      ReadPerCellResults(st, A, dt, stats, per_cell_status, per_cell_accepted);
+      return;
+    }
+    micmb_fused_config cfg = s.fused;
+    if (cfg.lu_in_shared && FusedWarpsPerCta(s, cfg) < 1)
+      cfg.lu_in_shared = 0;
+    const int warps = FusedWarpsPerCta(s, cfg);
+    if (warps < 1)
+      throw Error(MICMB_ERR_UNSUPPORTED, "mechanism too large for the fused kernel's shared-memory working set");
+    if (!s.dev.has_warp)
+      throw Error(MICMB_ERR_UNSUPPORTED, "mechanism exceeds the fused kernel's 16-bit table positions (nnz <= 65534)");
+    const bool lu_shared = cfg.lu_in_shared != 0;
+    WarpLayout W = MakeLayout(m.S, m.R, s.params.stages, (int32_t)m.info_rxn.size(), m.nnz, lu_shared);
+    const size_t smem = (size_t)W.per_warp * sizeof(double) * warps;
+    const int threads = warps * kWarp;
+    auto kernel = lu_shared ? k_fused<true> : k_fused<false>;
+    MICMB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int per_sm = 0;
+    MICMB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
+    if (per_sm < 1)
+      throw Error(MICMB_ERR_UNSUPPORTED, "fused kernel cannot be resident with this configuration");
+    if (cfg.ctas_per_sm > 0)
+      per_sm = std::min(per_sm, cfg.ctas_per_sm);
+    int64_t grid = (int64_t)per_sm * s.sm_count;
+    grid = std::max<int64_t>(1, std::min<int64_t>(grid, (n + warps - 1) / warps));
+
+    FusedArgs A = PerCellArgs(st, adj, n);
+    if (!lu_shared)
+    {
+      const int64_t slots = grid * warps;
+      const int64_t stride = ((int64_t)m.nnz + 1 + 31) & ~31ll;
+      if (st.lu_slot_count < slots * stride || !st.lu_slots.p)
+      {
+        st.lu_slots = DeviceMemory(sizeof(double) * (size_t)(slots * stride));
+        st.lu_slot_count = slots * stride;
+      }
+      A.lu_global = st.lu_slots.as<double>();
+      A.lu_slot_stride = stride;
+    }
+    if (n > 0 && !m.constraints.empty())
+    {
+      // algebraic constraints: the one-cell-per-thread kernel is the fused form that has them
+      if (adj)
+        throw Error(MICMB_ERR_UNSUPPORTED, "the adjoint does not cover algebraic constraints");
+      if (!SolveFusedThread(s, st, A, dt))
+        throw Error(MICMB_ERR_UNSUPPORTED, "one-cell-per-thread kernel cannot be resident");
+    }
+    else if (n > 0)
+    {
+      bool done = false;
+      if (s.fused.variant == 0)
+        done = SolveFusedStream(s, st, dt, A);
+      else if (s.fused.variant == 2)
+        done = SolveFusedThread(s, st, A, dt);
+      if (!done)
+      {
+        if (A.ckpt_k)
+          throw Error(MICMB_ERR_INTERNAL, "the direct fused kernel stores no stage vectors");
+        const StepBounds B = step_bounds(s.params, dt);
+        kernel<<<(unsigned)grid, threads, smem, st.stream>>>(s.dev, s.params, B, A, W);
+        MICMB_CUDA(cudaGetLastError());
+      }
+    }
+    ReadPerCellResults(st, A, dt, stats, per_cell_status, per_cell_accepted);
+  }
+
+  bool SolvePlainPerCellGroup(micmb_solver& s, micmb_state& st, double dt, micmb_solver_stats* stats,
+                              int32_t* per_cell_status, int32_t* per_cell_accepted)
+  {
+    if (st.n_cells < 1 || !GroupVariantApplies(s, st.n_cells))
+      return false;
+    const FusedArgs A = PerCellArgs(st, nullptr, st.n_cells);
+    SolveFusedGroup(s, st, A, dt);
+    ReadPerCellResults(st, A, dt, stats, per_cell_status, per_cell_accepted);
+    return true;
   }
 }  // namespace micmb

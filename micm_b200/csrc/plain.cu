@@ -751,6 +751,9 @@ namespace micmb
   void SolvePlain(micmb_solver& s, micmb_state& st, double dt, int32_t step_control, micmb_solver_stats* stats,
                   int32_t* per_cell_status, int32_t* per_cell_accepted)
   {
+    if (step_control == MICMB_STEP_GLOBAL ? SolveGlobalGroup(s, st, dt, stats, per_cell_status, per_cell_accepted)
+                                          : SolvePlainPerCellGroup(s, st, dt, stats, per_cell_status, per_cell_accepted))
+      return;
     EnsurePlainBuffers(st);
     const auto& m = *s.mech;
     const DevParams P = s.params;

@@ -2,11 +2,13 @@
 #pragma once
 
 #include "device.cuh"
+#include "group.cuh"
 #include "mechanism.hpp"
 
 #include <cuda_runtime.h>
 
 #include <memory>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <utility>
@@ -85,6 +87,18 @@ namespace micmb
                                  // or null (one-cell-per-thread variant only)
     int32_t max_ckpt;
   };
+
+  // cells per block and warps of the cell-group kernels
+  struct GroupChoice
+  {
+    int32_t G, W;
+  };
+  struct GroupTables
+  {
+    GroupChoice choice;
+    DeviceMemory memory;
+    DevGroup dev;
+  };
 }  // namespace micmb
 
 struct micmb_solver
@@ -104,6 +118,8 @@ struct micmb_solver
   micmb::DeviceMemory stream_block_bytes;  // [n_blocks]
   micmb::DeviceMemory stream_coef;         // StreamProgram coef_table
   int32_t n_stream_coef = 0;
+  std::mutex group_mutex;  // guards `group`: states of one solver may be solved from several threads
+  std::vector<std::unique_ptr<micmb::GroupTables>> group;
   int64_t adjoint_memory_limit = 0;  // bytes of adjoint checkpoints (0 = from free device memory)
 };
 
@@ -129,6 +145,8 @@ struct micmb_state
   // fused path
   micmb::DeviceMemory lu_slots;
   int64_t lu_slot_count = 0;  // doubles allocated in lu_slots
+  micmb::DeviceMemory group_ws;   // cell-group kernels: the cells' vectors outside shared memory
+  micmb::DeviceMemory group_ynew, group_err, group_ctl;  // plain method on them: Ynew, error sums, control
   micmb::DeviceMemory thread_ws;  // one-cell-per-thread variant: per-thread working sets
   micmb::DeviceMemory attempt_order;  // streamed kernel: block order of one attempt
   std::vector<int32_t> attempt_order_host;  // what attempt_order holds
@@ -215,6 +233,19 @@ namespace micmb
   bool StreamVariantApplies(const micmb_solver& s);
   // one cell per thread, working sets in global memory
   bool SolveFusedThread(micmb_solver& s, micmb_state& st, const FusedArgs& A, double dt);
+  // cell-group kernels: the block shape for n_cells cells, its work lists on the
+  // device, dynamic shared memory, resident blocks (0: the cells do not fit)
+  GroupChoice ChooseGroup(const micmb_solver& s, int64_t n_cells);
+  const GroupTables& GroupTablesFor(micmb_solver& s, const GroupChoice& choice);
+  size_t GroupSharedBytes(const micmb_solver& s, const GroupChoice& choice);
+  int GroupBlocksPerSm(const micmb_solver& s, const void* kernel, const GroupChoice& choice);
+  bool GroupVariantApplies(const micmb_solver& s, int64_t n_cells);
+  void SolveFusedGroup(micmb_solver& s, micmb_state& st, const FusedArgs& A, double dt);
+  // the plain method on them: per cell, or one step size for all cells; false: not taken
+  bool SolvePlainPerCellGroup(micmb_solver& s, micmb_state& st, double dt, micmb_solver_stats* stats,
+                              int32_t* per_cell_status, int32_t* per_cell_accepted);
+  bool SolveGlobalGroup(micmb_solver& s, micmb_state& st, double dt, micmb_solver_stats* stats,
+                        int32_t* per_cell_status, int32_t* per_cell_accepted);
   int StreamWarpsPerCta(const micmb_solver& s, int slots, int cap, bool lu_shared);
   // discrete adjoint sweep over the checkpoints of a fused solve of cells
   // [begin, begin + count) (begin a multiple of L; checkpoints hold those cells only)

@@ -1,0 +1,79 @@
+"""The cell-group kernels (working sets in shared memory, several warps and
+cells per block) against the one-cell-per-thread kernel, which runs the same
+sums in the same order: bit for bit, over the block shapes that the cell count
+and the mechanism's size select (one cell per block up to a lane per cell),
+ragged last groups, vector lengths that split a block's cells, every tableau,
+and cells whose state is not finite."""
+import numpy as np
+import pytest
+
+from micm_b200 import Solver, micm_bench, synthetic
+from gpu_helpers import make_state
+
+pytestmark = pytest.mark.gpu
+
+CASES = {  # mechanism, inputs(n), dt
+    "readme": (synthetic.readme_mechanism,
+               lambda m, n: synthetic.cell_inputs(m, n, 3, readme_foo=(1.0, 30.0)), 500.0),
+    "chapman": (lambda: micm_bench.mechanism("chapman"), lambda m, n: micm_bench.inputs("chapman", n, seed=4), 30.0),
+    "c60": (synthetic.CONFIGS["c60_adjoint"]["mech"],
+            lambda m, n: synthetic.cell_inputs(m, n, 5, t_range=(200.0, 310.0), night_fraction=0.5), 600.0),
+    "c210": (synthetic.CONFIGS["c210"]["mech"],
+             lambda m, n: synthetic.cell_inputs(m, n, 6, t_range=(200.0, 310.0), night_fraction=0.5), 60.0),
+}
+
+
+def _solve(solver, inp, dt, method, control):
+    st = make_state(solver, inp)
+    solver.update_state_parameters(st)
+    res = solver.solve(dt, st, method=method, step_control=control, per_cell=True)
+    st.sync_outputs_to_host()
+    return st.concentrations(), res
+
+
+# 1: one cell; 2 and 149: fewer cells than two per SM; 299, 1201 and 5000: groups
+# of 2, 4-8 and (tiny mechanisms) 32 cells, the last one ragged
+@pytest.mark.parametrize("name,n,L,stages", [
+    ("readme", 1, 1, 2), ("readme", 10007, 32, 3), ("chapman", 149, 100, 3), ("chapman", 5000, 8, 60),
+    ("c60", 1, 128, 4), ("c60", 299, 7, 4), ("c60", 1201, 32, 3), ("c60", 5000, 100, 40),
+    ("c210", 2, 1, 4), ("c210", 299, 3, 60), ("c210", 1201, 128, 2)])
+def test_group_kernels_equal_thread_kernel(cuda_device, name, n, L, stages):
+    make, inputs, dt = CASES[name]
+    mech = make()
+    inp = inputs(mech, n)
+    ref = Solver(mech, stages, vector_length=L)
+    ref.set_fused_config(variant=2, lu_in_shared=0, ctas_per_sm=5)
+    y_ref, r_ref = _solve(ref, inp, dt, "fused", "per_cell")
+    for method in ("fused", "plain"):
+        y, r = _solve(Solver(mech, stages, vector_length=L), inp, dt, method, "per_cell")
+        np.testing.assert_array_equal(y, y_ref)
+        np.testing.assert_array_equal(r.per_cell_status, r_ref.per_cell_status)
+        np.testing.assert_array_equal(r.per_cell_accepted, r_ref.per_cell_accepted)
+        assert r.stats == r_ref.stats
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -1.0e-9])
+def test_cells_that_are_not_finite(cuda_device, bad):
+    """A NaN, infinite or negative value stays in its own cell."""
+    make, inputs, dt = CASES["c60"]
+    mech, n = make(), 700
+    inp = inputs(mech, n)
+    inp["concentrations"][[0, 5, 333, 699], 7] = bad
+    ref = Solver(mech, 4, vector_length=32)
+    ref.set_fused_config(variant=2, lu_in_shared=0, ctas_per_sm=5)
+    y_ref, r_ref = _solve(ref, inp, dt, "fused", "per_cell")
+    y, r = _solve(Solver(mech, 4, vector_length=32), inp, dt, "fused", "per_cell")
+    np.testing.assert_array_equal(y, y_ref)
+    np.testing.assert_array_equal(r.per_cell_status, r_ref.per_cell_status)
+    assert r.stats == r_ref.stats
+
+
+def test_one_cell_global_equals_per_cell(cuda_device):
+    """With one cell the single step size is the cell's own."""
+    make, inputs, dt = CASES["c210"]
+    mech = make()
+    inp = inputs(mech, 1)
+    y_p, r_p = _solve(Solver(mech, 4, vector_length=8), inp, dt, "plain", "per_cell")
+    y_g, r_g = _solve(Solver(mech, 4, vector_length=8), inp, dt, "plain", "global")
+    np.testing.assert_array_equal(y_g, y_p)
+    assert r_g.stats["accepted"] == r_p.stats["accepted"] and r_g.stats["rejected"] == r_p.stats["rejected"]
