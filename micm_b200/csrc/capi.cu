@@ -82,6 +82,19 @@ namespace micmb
       d.c[i] = p.c[i];
     }
     d.inv_order = 1 / p.estimator_of_local_order;
+    // safety / error^(1 / order) decreases with the error: where it is past a
+    // clamp by more than any rounding, the clamp is the step-size factor and the
+    // power (8,500 cycles in double-double) need not be formed
+    d.error_lo = -1.0;
+    d.error_hi = INFINITY;
+    const double order = p.estimator_of_local_order;
+    if (p.safety_factor > 0 && p.factor_min > 0 && p.factor_max > p.factor_min && std::isfinite(p.factor_max) &&
+        std::isfinite(p.safety_factor) && order >= 1 && order <= 16)
+    {
+      constexpr double margin = 1e-9;
+      d.error_lo = std::pow(p.safety_factor / (p.factor_max * (1 + margin)), order) * (1 - margin);
+      d.error_hi = std::pow(p.safety_factor / (p.factor_min * (1 - margin)), order) * (1 + margin);
+    }
     d.gamma0 = p.gamma[0];
     d.cinit_max_iter = p.constraint_init_max_iterations;
     d.cinit_tol = p.constraint_init_tolerance;

@@ -132,6 +132,8 @@ namespace micmb
     int32_t new_f[6];
     double inv_order;  // 1 / estimator_of_local_order
     double a[15], c[15], m[6], e[6], gamma0;
+    // errors up to error_lo certainly give factor_max, from error_hi on factor_min
+    double error_lo, error_hi;
     int32_t cinit_max_iter;  // DAE constraint initialisation
     double cinit_tol;
   };
@@ -976,9 +978,17 @@ namespace micmb
   {
     // std::min(factor_max, std::max(factor_min, safety / pow(error, 1/order))),
     // with micm's (the C library's) correctly rounded pow
-    const double x = p.safety_factor / cr_pow(error, p.inv_order);
-    const double lo = (p.factor_min < x) ? x : p.factor_min;
-    const double fac = (lo < p.factor_max) ? lo : p.factor_max;
+    double fac;
+    if (error <= p.error_lo)
+      fac = p.factor_max;
+    else if (error >= p.error_hi)
+      fac = p.factor_min;
+    else
+    {
+      const double x = p.safety_factor / cr_pow(error, p.inv_order);
+      const double lo = (p.factor_min < x) ? x : p.factor_min;
+      fac = (lo < p.factor_max) ? lo : p.factor_max;
+    }
     double Hnew = c.H * fac;
     c.number_of_steps += 1;
     if (isnan(error))

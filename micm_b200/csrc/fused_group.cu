@@ -36,7 +36,7 @@ namespace micmb
     constexpr int32_t kSlotNothing = 6;   // a new cell that needs no step
 
     template<int G>
-    __global__ void k_group_solve(DevGroup P, DevParams D, StepBounds B, FusedArgs A, double* ws, int64_t slot_doubles)
+    __global__ void __launch_bounds__(256, 1) k_group_solve(DevGroup P, DevParams D, StepBounds B, FusedArgs A, double* ws, int64_t slot_doubles)
     {
       extern __shared__ __align__(16) double shared[];
       __shared__ CellCtl ctl[G];
@@ -146,7 +146,7 @@ namespace micmb
           if (threadIdx.x < G)
           {
             if (w == kSlotFresh)
-              what[g] = kSlotAccepted;  // its step starts with a new forcing
+              what[g] = kSlotAccepted;
             else if (w == kSlotNothing)
             {
               retire();
@@ -159,8 +159,7 @@ namespace micmb
         const bool live = w != kSlotIdle;
         if (!__syncthreads_or(live))
           break;
-        const bool new_f0 = __syncthreads_or(w == kSlotAccepted);
-        group_attempt<G>(P, D, X, v, ctl[g].H, new_f0, A.atol, A.rtol);
+        group_attempt<G>(P, D, X, v, ctl[g].H, A.atol, A.rtol);
         __syncthreads();
         if (threadIdx.x < G && live)
         {
@@ -309,7 +308,7 @@ namespace micmb
     auto phase = [&](const Offsets& o) {
       DevGroupPhase d;
       d.warp_start = reinterpret_cast<const int32_t*>(b + o.ws);
-      d.ctrl = reinterpret_cast<const uint4*>(b + o.ctrl);
+      d.ctrl = reinterpret_cast<const uint32_t*>(b + o.ctrl);
       d.item = reinterpret_cast<const uint4*>(b + o.item);
       d.row = reinterpret_cast<const uint4*>(b + o.row);
       d.coef = reinterpret_cast<const double2*>(b + o.coef);

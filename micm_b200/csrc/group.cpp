@@ -2,40 +2,37 @@
 #include "group.hpp"
 
 #include <algorithm>
+#include <map>
 #include <stdexcept>
 
 namespace micmb
 {
   namespace
   {
-    struct Unit
+    struct Sum
     {
       int32_t target, aux, kind;
-      std::vector<uint32_t> term;  // elements: pairs of operands, or gathered values
+      std::vector<uint32_t> term;  // operands a | b << 16, or a gathered value's element
       std::vector<double> coef;
-      int32_t n_terms(bool gather) const
-      {
-        return (int32_t)term.size() / (gather ? 1 : 2);
-      }
     };
 
     struct Chunk
     {
-      std::vector<const Unit*> units;
+      std::vector<const Sum*> units;
       int32_t T = 0, kind = 0;
     };
 
     // the units of one level in chunks of ipw, longest first within each kind
-    std::vector<Chunk> Cut(const std::vector<Unit>& units, int32_t ipw, bool gather)
+    std::vector<Chunk> Cut(const std::vector<Sum>& units, int32_t ipw)
     {
-      std::vector<const Unit*> order;
-      for (const Unit& u : units)
+      std::vector<const Sum*> order;
+      for (const Sum& u : units)
         order.push_back(&u);
-      std::stable_sort(order.begin(), order.end(), [](const Unit* a, const Unit* b) {
+      std::stable_sort(order.begin(), order.end(), [](const Sum* a, const Sum* b) {
         return a->kind != b->kind ? a->kind < b->kind : a->term.size() > b->term.size();
       });
       std::vector<Chunk> chunks;
-      for (const Unit* u : order)
+      for (const Sum* u : order)
       {
         if (chunks.empty() || (int32_t)chunks.back().units.size() == ipw || chunks.back().kind != u->kind)
         {
@@ -43,20 +40,56 @@ namespace micmb
           chunks.back().kind = u->kind;
         }
         chunks.back().units.push_back(u);
-        chunks.back().T = std::max<int32_t>(chunks.back().T, u->n_terms(gather));
+        chunks.back().T = std::max<int32_t>(chunks.back().T, (int32_t)u->term.size());
       }
       return chunks;
     }
 
-    // Chunk lists of all warps while a phase is being built.
+    // One unit: up to four chunks, or terms [t0, t0 + 16) of one.
+    struct Step
+    {
+      std::vector<Chunk> chunks;
+      int32_t t0 = 0;
+      bool first = true, last = true;
+      int32_t sync = kGroupNoSync;
+    };
+
+    // The chunks of one level, longest first within each kind, as units; a long
+    // chunk's units stay together.
+    std::vector<std::vector<Step>> Pack(const std::vector<Chunk>& chunks)
+    {
+      std::vector<std::vector<Step>> out;
+      for (size_t i = 0; i < chunks.size();)
+      {
+        const int32_t T = chunks[i].T, kind = chunks[i].kind;
+        out.emplace_back();
+        if (T > kGroupTerms / 2)
+        {
+          for (int32_t t0 = 0; t0 < T; t0 += kGroupTerms)
+          {
+            Step st;
+            st.chunks = { chunks[i] };
+            st.t0 = t0;
+            st.first = t0 == 0;
+            st.last = t0 + kGroupTerms >= T;
+            out.back().push_back(std::move(st));
+          }
+          ++i;
+          continue;
+        }
+        Step st;
+        const size_t most = T > kGroupTerms / 4 ? 2 : 4;
+        for (; i < chunks.size() && st.chunks.size() < most && chunks[i].kind == kind; ++i)
+          st.chunks.push_back(chunks[i]);
+        out.back().push_back(std::move(st));
+      }
+      return out;
+    }
+
+    // Unit lists of all warps while a phase is being built.
     struct Lists
     {
-      struct Entry
-      {
-        Chunk chunk;
-        int32_t sync;
-      };
-      std::vector<std::vector<Entry>> warp;
+      std::vector<std::vector<Step>> warp;
 
       explicit Lists(int32_t W)
           : warp(W)
@@ -68,111 +101,165 @@ namespace micmb
         for (auto& list : warp)
         {
           if (list.empty() || list.back().sync == kGroupBlockSync)
-            list.push_back({ Chunk{}, kGroupNoSync });
+            list.emplace_back();  // nothing but the barrier
           list.back().sync = kGroupBlockSync;
         }
       }
+
+      void Append(size_t w, std::vector<Step> steps)
+      {
+        for (Step& st : steps)
+          warp[w].push_back(std::move(st));
+      }
     };
 
-    // Longest chunk first onto the least loaded warp.  The cost of a chunk is
-    // about its fixed part (descriptor, item, first load, store) plus its terms.
-    void Deal(Lists& lists, std::vector<Chunk> chunks)
+    // longest first onto the least loaded warp
+    void Deal(Lists& lists, std::vector<std::vector<Step>> packed)
     {
-      std::stable_sort(chunks.begin(), chunks.end(), [](const Chunk& a, const Chunk& b) { return a.T > b.T; });
-      std::vector<int64_t> load(lists.warp.size(), 0);
-      for (Chunk& c : chunks)
+      std::stable_sort(packed.begin(), packed.end(), [](const auto& a, const auto& b) { return a.size() > b.size(); });
+      std::vector<size_t> load(lists.warp.size(), 0);
+      for (auto& steps : packed)
       {
         const size_t w = (size_t)(std::min_element(load.begin(), load.end()) - load.begin());
-        load[w] += 4 + c.T;
-        lists.warp[w].push_back({ std::move(c), kGroupNoSync });
+        load[w] += steps.size();
+        lists.Append(w, std::move(steps));
       }
     }
 
-    void Emit(GroupPhase& ph, const Lists& lists, const GroupLayout& L, int32_t G, bool gather)
+    // pivot_is_aux: kGroupPivot writes aux (the LU)
+    void Emit(GroupPhase& ph, const Lists& lists, const GroupLayout& L, int32_t G, bool gather,
+              bool pivot_is_aux = false)
     {
       const int32_t ipw = 32 / G;
-      auto offset = [&](int32_t e) { return (uint32_t)e * (uint32_t)G * 8u; };
-      std::vector<std::vector<uint32_t>> items;  // per record, [lane][words]
-      const int32_t item_words = gather ? 1 : 2;
-      auto record = [&](const Chunk& c, int32_t t0, uint32_t ctrl) {
-        ph.ctrl.push_back(ctrl);
-        items.emplace_back();
-        auto unit = [&](int32_t p) { return p < (int32_t)c.units.size() ? c.units[p] : nullptr; };
+      auto emit = [&](const Step& st) {
+        int32_t T = 0;
+        for (const Chunk& c : st.chunks)
+          T = std::max(T, std::min(kGroupTerms, c.T - st.t0));
+        uint32_t shape = 0;
+        while (kGroupShapes[shape].chunks < (int32_t)st.chunks.size() || kGroupShapes[shape].terms < T)
+          ++shape;
+        if (!st.first || !st.last)
+          shape = 2;  // stretches of a long sum
+        const int32_t per_chunk = kGroupTerms / kGroupShapes[shape].chunks;
+        const int32_t kind = st.chunks.empty() ? kGroupPlain : st.chunks[0].kind;
+        ph.ctrl.push_back((shape * 3 + (uint32_t)(st.last ? kind : kGroupNone)) | (uint32_t)st.sync << 8 |
+                          (st.first ? 1u << 10 : 0u));
+        auto unit = [&](int32_t k, int32_t p) -> const Sum* {
+          return k < (int32_t)st.chunks.size() && p < (int32_t)st.chunks[k].units.size() ? st.chunks[k].units[p]
+                                                                                         : nullptr;
+        };
         for (int32_t p = 0; p < ipw; ++p)
-        {
-          const Unit* u = unit(p);
-          if (gather)
-            items.back().push_back(u ? (uint32_t)u->target | ((uint32_t)u->aux << 16) : kGroupNoItem);
-          else
+          for (int32_t k = 0; k < 4; ++k)
           {
-            items.back().push_back(offset(u ? u->target : L.trash));
-            items.back().push_back(offset(u ? u->aux : (c.kind == kGroupRecip ? L.trash : L.one)));
+            const Sum* u = unit(k, p);
+            const uint32_t idle = (uint32_t)L.trash |
+                                  (gather ? 0u : (uint32_t)(pivot_is_aux && kind == kGroupPivot ? L.trash : L.one) << 16);
+            ph.item.push_back(u ? (uint32_t)u->target | (uint32_t)u->aux << 16 : idle);
           }
-        }
-        auto term = [&](int32_t p, int32_t t, int32_t k) {
-          const Unit* u = unit(p);
-          return offset(u && t < u->n_terms(gather) ? (int32_t)u->term[gather ? t : 2 * t + k] : L.zero);
+        auto term = [&](int32_t p, int32_t t, double* coef) {
+          const Sum* u = unit(t / per_chunk, p);
+          const int32_t i = st.t0 + t % per_chunk;
+          const bool real = u && i < (int32_t)u->term.size();
+          if (coef)
+            *coef = real ? u->coef[i] : 0.0;
+          const uint32_t zero = (uint32_t)L.zero;
+          return real ? u->term[i] : (gather ? zero : zero | zero << 16);
         };
         if (gather)
         {
-          for (int32_t p = 0; p < ipw; ++p)
-            for (int32_t q = 0; q < 4; ++q)
-              ph.row.push_back(term(p, t0 + q, 0));
-          for (int32_t h = 0; h < 2; ++h)
+          for (int32_t r = 0; r < 2; ++r)
             for (int32_t p = 0; p < ipw; ++p)
-              for (int32_t q = 2 * h; q < 2 * h + 2; ++q)
+              for (int32_t t = 8 * r; t < 8 * r + 8; t += 2)
+                ph.row.push_back(term(p, t, nullptr) | term(p, t + 1, nullptr) << 16);
+          for (int32_t r = 0; r < 8; ++r)
+            for (int32_t p = 0; p < ipw; ++p)
+              for (int32_t t = 2 * r; t < 2 * r + 2; ++t)
               {
-                const Unit* u = unit(p);
-                ph.coef.push_back(u && t0 + q < u->n_terms(true) ? u->coef[t0 + q] : 0.0);
+                double c;
+                term(p, t, &c);
+                ph.coef.push_back(c);
               }
         }
         else
-          for (int32_t h = 0; h < 2; ++h)
+          for (int32_t r = 0; r < 4; ++r)
             for (int32_t p = 0; p < ipw; ++p)
-              for (int32_t q = 2 * h; q < 2 * h + 2; ++q)
-                for (int32_t k = 0; k < 2; ++k)
-                  ph.row.push_back(term(p, t0 + q, k));
+              for (int32_t t = 4 * r; t < 4 * r + 4; ++t)
+                ph.row.push_back(term(p, t, nullptr));
       };
       ph.warp_start.push_back(0);
       for (const auto& list : lists.warp)
       {
-        for (const auto& e : list)
-        {
-          const Chunk& c = e.chunk;
-          const int32_t n = std::max<int32_t>(1, (c.T + 3) / 4);
-          for (int32_t j = 0; j < n; ++j)
-          {
-            uint32_t ctrl = (uint32_t)std::min<int32_t>(4, c.T - 4 * j);
-            if (!c.units.empty())
-              ctrl |= (j == 0 ? 1u << 3 : 0u) | (j == n - 1 ? 1u << 4 : 0u) | ((uint32_t)c.kind << 5);
-            if (j == n - 1)
-              ctrl |= (uint32_t)e.sync << 7;
-            record(c, 4 * j, ctrl);
-          }
-        }
-        while (ph.ctrl.size() % kGroupUnit)
-          record(Chunk{}, 0, 0);
-        ph.warp_start.push_back((int32_t)(ph.ctrl.size() / kGroupUnit));
+        for (const Step& st : list)
+          emit(st);
+        ph.warp_start.push_back((int32_t)ph.ctrl.size());
       }
-      // fetched ahead, never run
-      for (int32_t j = 0; j < kGroupUnit; ++j)
-        record(Chunk{}, 0, 0);
-      for (size_t u = 0; u < ph.ctrl.size() / kGroupUnit; ++u)
-        for (int32_t p = 0; p < ipw; ++p)
-          for (int32_t j = 0; j < kGroupUnit; ++j)
-            for (int32_t k = 0; k < item_words; ++k)
-              ph.item.push_back(items[u * kGroupUnit + j][(size_t)p * item_words + k]);
+      emit(Step{});  // fetched ahead, never run
     }
 
-    // A level with at most this many chunks runs on the first warp alone, with
-    // warp synchronisation: a block barrier costs more than a second chunk.
-    constexpr int32_t kNarrowChunks = 2;
+    // One stretch of an item's terms, in the level where it runs.
+    struct Piece
+    {
+      int32_t level, item, t0, t1;
+      bool last;  // the item's value is final after it
+    };
 
-    // Chunk lists of one or more level schedules run one after the other.
+    // Dependency levels of a serial schedule.  Term t of an item can run one level
+    // after its operands are final (and after the item's earlier terms); an item
+    // is finished in the first level that has all of its terms.  Terms that are
+    // ready earlier run in batches of kBatch as they come (a stretch loads and
+    // stores the item's sum, so short stretches cost more than they do), the rest
+    // with the last ones.  Exact: the sum is only stored and reloaded in between.
+    constexpr int32_t kBatch = 4;
+    std::vector<std::vector<Piece>> Levels(const LevelSchedule& s, bool factor)
+    {
+      const int32_t n = s.n_items();
+      std::map<int32_t, int32_t> item_of;
+      for (int32_t i = 0; i < n; ++i)
+        item_of[s.item_target[i]] = i;
+      std::vector<int32_t> final_level(n, 0);
+      std::vector<std::vector<Piece>> levels;
+      auto put = [&](const Piece& p) {
+        if ((int32_t)levels.size() <= p.level)
+          levels.resize(p.level + 1);
+        levels[p.level].push_back(p);
+      };
+      for (int32_t i = 0; i < n; ++i)
+      {
+        const int32_t t0 = s.term_start[i], t1 = s.term_start[i + 1];
+        std::vector<int32_t> ready;
+        int32_t level = 0;
+        for (int32_t t = t0; t < t1; ++t)
+        {
+          if (factor)
+            level = std::max(level, final_level[item_of.at(s.term_a[t])] + 1);
+          level = std::max(level, final_level[item_of.at(s.term_b[t])] + 1);
+          ready.push_back(level);
+        }
+        // an L entry's scaling needs its pivot
+        if (factor && s.item_aux[i] >= 0)
+          level = std::max(level, final_level[item_of.at(s.item_aux[i])] + 1);
+        final_level[i] = level;
+        int32_t start = 0;
+        for (int32_t t = 0; t < t1 - t0; ++t)
+          if (ready[t] < level && t + 1 - start >= kBatch && (t + 1 == t1 - t0 || ready[t + 1] > ready[t]))
+          {
+            put({ ready[t], i, t0 + start, t0 + t + 1, false });
+            start = t + 1;
+          }
+        put({ level, i, t0 + start, t1, true });
+      }
+      return levels;
+    }
+
+    // A level with at most this many units runs on the first warp alone, with
+    // warp synchronisation: a block barrier costs more than a second unit.
+    constexpr size_t kNarrowUnits = 2;
+
+    // Unit lists of one or more level schedules run one after the other.
     struct LevelLists
     {
       Lists lists;
-      std::vector<std::vector<Unit>> kept;  // the chunks point into them
+      std::vector<std::vector<Sum>> kept;  // the chunks point into them
       bool narrow_run = false;
 
       explicit LevelLists(int32_t W)
@@ -180,25 +267,28 @@ namespace micmb
       {
       }
 
-      template<class MakeUnit>
-      void Add(const LevelSchedule& s, int32_t ipw, MakeUnit make)
+      template<class MakeSum>
+      void Add(const LevelSchedule& s, bool factor, int32_t ipw, int32_t one, MakeSum make)
       {
-        for (int32_t l = 0; l < s.n_levels(); ++l)
+        for (const std::vector<Piece>& pieces : Levels(s, factor))
         {
-          std::vector<Unit> units;
-          for (int32_t i = s.level_start[l]; i < s.level_start[l + 1]; ++i)
+          std::vector<Sum> units;
+          for (const Piece& piece : pieces)
           {
-            Unit u = make(i);
+            Sum u = make(piece);
             // an item without terms that keeps its value has nothing to do
-            if (u.term.empty() && u.kind == kGroupStore)
+            if (u.term.empty() && u.kind == kGroupPlain && u.aux == one)
               continue;
             units.push_back(std::move(u));
           }
-          kept.push_back(std::move(units));
-          std::vector<Chunk> chunks = Cut(kept.back(), ipw, false);
-          if (chunks.empty())
+          if (units.empty())
             continue;
-          const bool narrow = lists.warp.size() == 1 || (int32_t)chunks.size() <= kNarrowChunks;
+          kept.push_back(std::move(units));
+          std::vector<std::vector<Step>> packed = Pack(Cut(kept.back(), ipw));
+          size_t n_units = 0;
+          for (const auto& steps : packed)
+            n_units += steps.size();
+          const bool narrow = lists.warp.size() == 1 || n_units <= kNarrowUnits;
           if (!lists.warp[0].empty())
           {
             if (narrow && narrow_run)
@@ -207,35 +297,36 @@ namespace micmb
               lists.BlockSync();
           }
           if (narrow)
-            for (Chunk& c : chunks)
-              lists.warp[0].push_back({ std::move(c), kGroupNoSync });
+            for (auto& steps : packed)
+              lists.Append(0, std::move(steps));
           else
-            Deal(lists, std::move(chunks));
+            Deal(lists, std::move(packed));
           narrow_run = narrow;
         }
       }
     };
 
+    // sums of coef * (element src0 + src) into elements target0 + i; flag: adds alpha
     GroupPhase GatherPhase(const std::vector<int32_t>& start, const std::vector<int32_t>& src,
-                           const std::vector<double>& coef, int32_t src0, const GroupLayout& L, int32_t G, int32_t W,
-                           const std::vector<char>& flag)
+                           const std::vector<double>& coef, int32_t src0, int32_t target0, const GroupLayout& L,
+                           int32_t G, int32_t W, const std::vector<char>& flag)
     {
-      std::vector<Unit> units;
+      std::vector<Sum> sums;
       for (int32_t i = 0; i + 1 < (int32_t)start.size(); ++i)
       {
-        Unit u;
-        u.target = i;
+        Sum u;
+        u.target = target0 + i;
         u.aux = flag.empty() ? 0 : flag[i];
-        u.kind = kGroupScale;
+        u.kind = kGroupPlain;
         for (int32_t t = start[i]; t < start[i + 1]; ++t)
         {
           u.term.push_back((uint32_t)(src0 + src[t]));
           u.coef.push_back(coef[t]);
         }
-        units.push_back(std::move(u));
+        sums.push_back(std::move(u));
       }
       Lists lists(W);
-      Deal(lists, Cut(units, 32 / G, true));
+      Deal(lists, Pack(Cut(sums, 32 / G)));
       GroupPhase ph;
       Emit(ph, lists, L, G, true);
       return ph;
@@ -252,8 +343,8 @@ namespace micmb
     L.trash = L.v0 + m.S;
     L.w0 = L.trash + 1;
     L.inv = L.w0;
-    L.rate = L.w0 + m.S;
-    L.elements = L.w0 + std::max(n_info, m.S + std::max(m.R, m.S));
+    L.rate = L.inv + m.S + 1;
+    L.elements = L.w0 + std::max(n_info, m.S + 1 + std::max(m.R, m.S));
     return L;
   }
 
@@ -288,37 +379,37 @@ namespace micmb
       P.drate.push_back(vec(d[2]) | (vec(d[3]) << 16));
     }
 
-    P.forcing = GatherPhase(m.f_start, m.f_rxn, m.f_coef, L.rate, L, G, W, {});
+    P.forcing = GatherPhase(m.f_start, m.f_rxn, m.f_coef, L.rate, L.v0, L, G, W, {});
     std::vector<char> diag(m.nnz, 0);
     for (int32_t i = 0; i < m.S; ++i)
       diag[m.diag_pos[i]] = 1;
-    P.jacobian = GatherPhase(m.j_start, m.j_info, m.j_coef, L.w0, L, G, W, diag);
+    P.jacobian = GatherPhase(m.j_start, m.j_info, m.j_coef, L.w0, 0, L, G, W, diag);
 
     LevelLists lu(W);
-    lu.Add(m.lu, ipw, [&](int32_t i) {
-      Unit u;
-      u.target = m.lu.item_target[i];
-      const bool partial = m.lu.item_aux[i] == -2;
+    lu.Add(m.lu_serial, true, ipw, L.one, [&](const Piece& p) {
+      Sum u;
+      u.target = m.lu_serial.item_target[p.item];
       const int32_t row = m.nz_row[u.target], col = m.nz_col[u.target];
-      // scaling by one keeps partial sums and U entries in the chunks of the L entries
-      u.kind = partial || row < col ? (m.lu.term_start[i] == m.lu.term_start[i + 1] ? kGroupStore : kGroupScale)
-                                    : (row == col ? kGroupRecip : kGroupScale);
-      u.aux = partial || row < col ? L.one : L.inv + (row == col ? row : col);
-      for (int32_t t = m.lu.term_start[i]; t < m.lu.term_start[i + 1]; ++t)
-        u.term.insert(u.term.end(), { (uint32_t)m.lu.term_a[t], (uint32_t)m.lu.term_b[t] });
+      const bool scaled = p.last && row > col;
+      // partial sums and U entries share the units of the L entries: scaled by one
+      u.kind = p.last && row == col ? kGroupPivot : kGroupPlain;
+      u.aux = scaled ? L.inv + col : (u.kind == kGroupPivot ? L.inv + row : L.one);
+      for (int32_t t = p.t0; t < p.t1; ++t)
+        u.term.push_back((uint32_t)m.lu_serial.term_a[t] | (uint32_t)m.lu_serial.term_b[t] << 16);
       return u;
     });
-    Emit(P.lu, lu.lists, L, G, false);
+    Emit(P.lu, lu.lists, L, G, false, true);
 
     LevelLists solve(W);
-    for (const LevelSchedule* s : { &m.fwd, &m.bwd })
-      solve.Add(*s, ipw, [&](int32_t i) {
-        Unit u;
-        u.target = L.v0 + s->item_target[i];
-        u.kind = s->item_aux[i] >= 0 ? kGroupDiv : kGroupStore;
-        u.aux = s->item_aux[i] >= 0 ? s->item_aux[i] : L.one;
-        for (int32_t t = s->term_start[i]; t < s->term_start[i + 1]; ++t)
-          u.term.insert(u.term.end(), { (uint32_t)s->term_a[t], (uint32_t)(L.v0 + s->term_b[t]) });
+    for (const LevelSchedule* s : { &m.fwd_serial, &m.bwd_serial })
+      solve.Add(*s, false, ipw, L.one, [&](const Piece& p) {
+        Sum u;
+        u.target = L.v0 + s->item_target[p.item];
+        const bool divided = p.last && s->item_aux[p.item] >= 0;
+        u.kind = divided ? kGroupPivot : kGroupPlain;
+        u.aux = divided ? s->item_aux[p.item] : L.one;
+        for (int32_t t = p.t0; t < p.t1; ++t)
+          u.term.push_back((uint32_t)s->term_a[t] | (uint32_t)(L.v0 + s->term_b[t]) << 16);
         return u;
       });
     Emit(P.solve, solve.lists, L, G, false);

@@ -14,10 +14,10 @@ namespace micmb
   struct DevGroupPhase
   {
     const int32_t* warp_start;
-    const uint4* ctrl;    // per unit
-    const uint4* item;    // per unit and lane: two (level phases) or one (gathers)
-    const uint4* row;     // per record and lane: two (level phases) or one (gathers)
-    const double2* coef;  // gathers: two per record and lane
+    const uint32_t* ctrl;  // per unit
+    const uint4* item;     // per unit and lane
+    const uint4* row;      // per unit and lane: four (level phases) or two (gathers)
+    const double2* coef;   // gathers: eight per unit and lane
   };
 
   struct DevGroup
@@ -29,11 +29,14 @@ namespace micmb
     const uint2* drate_tab;
   };
 
-  // one thread's view of its cell
+  // One thread's view of its cell.  The table-driven loops address shared memory
+  // by 32-bit addresses formed in one instruction from a 16-bit element index
+  // (dp2a: base + index * 8 G).
   template<int G>
   struct GroupThread
   {
     double* s;      // element e at s[e * G]
+    uint32_t base;  // its shared-memory address
     int32_t lane;   // item lane in the block
     int32_t lanes;  // item lanes of the block
     int32_t warp;   // warp in the block
@@ -41,6 +44,7 @@ namespace micmb
 
     __device__ __forceinline__ explicit GroupThread(double* shared)
         : s(shared + (threadIdx.x & (G - 1))),
+          base((uint32_t)__cvta_generic_to_shared(s)),
           lane((int32_t)(threadIdx.x / G)),
           lanes((int32_t)(blockDim.x / G)),
           warp(__shfl_sync(0xffffffffu, (int32_t)(threadIdx.x >> 5), 0)),  // known to be the warp's
@@ -51,10 +55,30 @@ namespace micmb
     {
       return s[e * G];
     }
-    // element at a byte offset of the tables
-    __device__ __forceinline__ double& at(uint32_t offset) const
+    // addresses of the elements in a table word's halves
+    __device__ __forceinline__ uint32_t lo(uint32_t w) const
     {
-      return *reinterpret_cast<double*>(reinterpret_cast<char*>(s) + offset);
+      if constexpr (G * 8 < 256)
+        return __dp2a_lo(w, (uint32_t)(G * 8), base);
+      else
+        return base + (w & 0xFFFFu) * (G * 8);
+    }
+    __device__ __forceinline__ uint32_t hi(uint32_t w) const
+    {
+      if constexpr (G * 8 < 256)
+        return __dp2a_lo(w, (uint32_t)(G * 8) << 8, base);
+      else
+        return base + (w >> 16) * (G * 8);
+    }
+    static __device__ __forceinline__ double load(uint32_t address)
+    {
+      double v;
+      asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(address) : "memory");
+      return v;
+    }
+    static __device__ __forceinline__ void store(uint32_t address, double v)
+    {
+      asm volatile("st.shared.f64 [%0], %1;" ::"r"(address), "d"(v) : "memory");
     }
   };
 
@@ -65,175 +89,254 @@ namespace micmb
   // within the ulp.  Five dependent operations where the divide takes about 110
   // cycles; operands whose exponents could leave the normal range anywhere on
   // the way (zeros, infinities and NaN among them) take the divide.
-  __device__ __forceinline__ double divide_by(double v, double d, double r)
+  static __device__ __noinline__ double divide_slowly(double v, double d)
   {
-    const int32_t ev = (__double2hiint(v) >> 20) & 0x7FF, ed = (__double2hiint(d) >> 20) & 0x7FF;
-    if (v == 0.0 && (uint32_t)(ed - 523) <= 1000u)
-      return v * r;  // a zero with the quotient's sign
-    // exponents within 2^-500 .. 2^500
-    if ((uint32_t)(ev - 523) <= 1000u && (uint32_t)(ed - 523) <= 1000u)
-    {
-      double q = v * r;
-      q = fma(fma(-q, d, v), r, q);
-      return fma(fma(-q, d, v), r, q);
-    }
     return v / d;
   }
 
-  // The records of this warp in one level phase, a unit of four at a time: the
-  // next unit's table words are fetched (all together, so that they share one
-  // wait) while this one is worked on, across barriers, since nothing in them
-  // depends on the cells.  A unit takes a few hundred cycles, about what a
-  // fetch from L2 takes.
-  template<int G>
+  __device__ __forceinline__ double divide_by(double v, double d, double r)
+  {
+    double q = v * r;
+    q = fma(fma(-q, d, v), r, q);
+    q = fma(fma(-q, d, v), r, q);
+    const int32_t ev = (__double2hiint(v) >> 20) & 0x7FF, ed = (__double2hiint(d) >> 20) & 0x7FF;
+    // exponents within 2^-500 .. 2^500
+    if ((uint32_t)(ev - 523) > 1000u || (uint32_t)(ed - 523) > 1000u)
+      q = (v == 0.0 && (uint32_t)(ed - 523) <= 1000u) ? v * r  // a zero with the quotient's sign
+                                                      : divide_slowly(v, d);
+    return q;
+  }
+
+  // A unit's table words.
+  template<int G, bool LU>
+  struct LevelUnit
+  {
+    uint32_t ctrl;
+    uint4 item, row[4];
+
+    __device__ __forceinline__ void fetch(const uint32_t*& cp, const uint4*& ip, const uint4*& rp)
+    {
+      constexpr int ipw = 32 / G;
+      ctrl = __ldg(cp);
+      item = __ldg(ip);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        row[j] = __ldg(rp + j * ipw);
+      cp += 1;
+      ip += ipw;
+      rp += 4 * ipw;
+    }
+
+    __device__ __forceinline__ uint32_t item_word(int k) const
+    {
+      return k == 0 ? item.x : (k == 1 ? item.y : (k == 2 ? item.z : item.w));
+    }
+    __device__ __forceinline__ uint32_t term_word(int t) const
+    {
+      const uint4 q = row[t / 4];
+      return t % 4 == 0 ? q.x : (t % 4 == 1 ? q.y : (t % 4 == 2 ? q.z : q.w));
+    }
+
+    // The unit with C chunks of T terms; the chunks' sums run side by side.
+    template<int C, int T, int FIN>
+    __device__ __forceinline__ void run(const GroupThread<G>& X, uint32_t inv_offset, double& carry) const
+    {
+      double v[C], d[C], r[C];
+#pragma unroll
+      for (int k = 0; k < C; ++k)
+      {
+        v[k] = X.load(X.lo(item_word(k)));
+        if (FIN == (LU ? kGroupPlain : kGroupPivot))
+          d[k] = X.load(X.hi(item_word(k)));
+        if (!LU && FIN == kGroupPivot)
+          r[k] = X.load(X.lo(item_word(k)) + inv_offset);
+      }
+      if (C == 1 && T == 16 && !(ctrl & 1024u))
+        v[0] = carry;
+#pragma unroll
+      for (int t = 0; t < T; ++t)
+      {
+        double p[C];
+#pragma unroll
+        for (int k = 0; k < C; ++k)
+        {
+          const uint32_t w = term_word(k * (16 / C) + t);
+          const double a = X.load(X.lo(w)), b = X.load(X.hi(w));
+          p[k] = a * b;
+        }
+#pragma unroll
+        for (int k = 0; k < C; ++k)
+          v[k] -= p[k];
+      }
+      if (C == 1 && FIN == kGroupNone)
+        carry = v[0];
+      else
+#pragma unroll
+        for (int k = 0; k < C; ++k)
+        {
+          const uint32_t target = X.lo(item_word(k));
+          if (FIN == kGroupPlain)
+            X.store(target, LU ? v[k] * d[k] : v[k]);
+          else if (!LU)
+            X.store(target, divide_by(v[k], d[k], r[k]));
+          else
+          {
+            X.store(target, v[k]);
+            X.store(X.hi(item_word(k)), 1.0 / v[k]);
+          }
+        }
+    }
+
+    // one jump per unit: a taken branch costs a lone warp about 25 cycles
+    __device__ __forceinline__ void run(const GroupThread<G>& X, uint32_t inv_offset, double& carry) const
+    {
+#define MICMB_GROUP_CASES(shape, C, T)                        \
+  case shape * 3 + kGroupPlain: run<C, T, kGroupPlain>(X, inv_offset, carry); break; \
+  case shape * 3 + kGroupPivot: run<C, T, kGroupPivot>(X, inv_offset, carry); break;
+      switch (ctrl & 255u)
+      {
+        MICMB_GROUP_CASES(0, 1, 4)
+        MICMB_GROUP_CASES(1, 1, 8)
+        MICMB_GROUP_CASES(2, 1, 16)
+        MICMB_GROUP_CASES(3, 2, 4)
+        MICMB_GROUP_CASES(4, 2, 8)
+        MICMB_GROUP_CASES(5, 4, 2)
+        MICMB_GROUP_CASES(6, 4, 4)
+        case 2 * 3 + kGroupNone: run<1, 16, kGroupNone>(X, inv_offset, carry); break;
+      }
+#undef MICMB_GROUP_CASES
+      if (ctrl & (kGroupBlockSync << 8))
+        __syncthreads();
+      else
+        __syncwarp();
+    }
+  };
+
+  // The units of this warp in one level phase.  The next unit's table words are
+  // fetched while this one is worked on, across barriers, since nothing in them
+  // depends on the cells.  The copy waits for all of a unit's words before the
+  // next ones are asked for.
+  template<int G, bool LU>
   __device__ __forceinline__ void run_levels(const DevGroupPhase& ph, const GroupThread<G>& X, const DevGroup& P)
   {
-    constexpr int ipw = 32 / G, U = kGroupUnit;
+    constexpr int ipw = 32 / G;
     const uint32_t inv_offset = (uint32_t)(P.inv - P.v0) * (G * 8);
     int32_t u = ph.warp_start[X.warp];
     const int32_t u1 = ph.warp_start[X.warp + 1];
-    if (u == u1)
-      return;
-    const uint4* cp = ph.ctrl + u;
-    const uint4* ip = ph.item + ((int64_t)u * ipw + X.sub) * 2;
-    const uint4* rp = ph.row + (int64_t)u * (U * 2 * ipw) + X.sub;
-    uint4 nctrl = __ldg(cp), nitem[2] = { __ldg(ip), __ldg(ip + 1) }, nrow[2 * U];
-#pragma unroll
-    for (int j = 0; j < 2 * U; ++j)
-      nrow[j] = __ldg(rp + j * ipw);
-    double v = 0.0;
+    const uint32_t* cp = ph.ctrl + u;
+    const uint4* ip = ph.item + ((int64_t)u * ipw + X.sub);
+    const uint4* rp = ph.row + ((int64_t)u * (4 * ipw) + X.sub);
+    LevelUnit<G, LU> next;
+    double carry = 0.0;
+    if (u < u1)
+      next.fetch(cp, ip, rp);
+#pragma unroll 1
     for (; u < u1; ++u)
     {
-      const uint32_t ctrl[U] = { nctrl.x, nctrl.y, nctrl.z, nctrl.w };
-      const uint32_t target[U] = { nitem[0].x, nitem[0].z, nitem[1].x, nitem[1].z };
-      const uint32_t aux[U] = { nitem[0].y, nitem[0].w, nitem[1].y, nitem[1].w };
-      uint4 row[2 * U];
-#pragma unroll
-      for (int j = 0; j < 2 * U; ++j)
-        row[j] = nrow[j];
-      cp += 1;
-      ip += 2 * ipw;
-      rp += U * 2 * ipw;
-      nctrl = __ldg(cp);
-      nitem[0] = __ldg(ip);
-      nitem[1] = __ldg(ip + 1);
-#pragma unroll
-      for (int j = 0; j < 2 * U; ++j)
-        nrow[j] = __ldg(rp + j * ipw);
-#pragma unroll
-      for (int j = 0; j < U; ++j)
-      {
-        const uint32_t c = ctrl[j], T = c & 7u;
-        const uint4 a = row[2 * j], b = row[2 * j + 1];
-        if (c & 8u)
-          v = X.at(target[j]);
-        if (T > 2)
-        {
-          const double p0 = X.at(a.x) * X.at(a.y), p1 = X.at(a.z) * X.at(a.w);
-          const double p2 = X.at(b.x) * X.at(b.y), p3 = X.at(b.z) * X.at(b.w);
-          v -= p0;
-          v -= p1;
-          v -= p2;
-          v -= p3;
-        }
-        else if (T > 0)
-        {
-          const double p0 = X.at(a.x) * X.at(a.y), p1 = X.at(a.z) * X.at(a.w);
-          v -= p0;
-          v -= p1;
-        }
-        if (c & 16u)
-        {
-          const uint32_t kind = (c >> 5) & 3u;
-          if (kind == kGroupStore)
-            X.at(target[j]) = v;
-          else if (kind == kGroupScale)
-            X.at(target[j]) = v * X.at(aux[j]);
-          else if (kind == kGroupDiv)
-            X.at(target[j]) = divide_by(v, X.at(aux[j]), X.at(target[j] + inv_offset));
-          else
-          {
-            X.at(target[j]) = v;
-            X.at(aux[j]) = 1.0 / v;
-          }
-        }
-        const uint32_t sync = c >> 7;
-        if (sync == 2)
-          __syncthreads();
-        else if (sync == 1)
-          __syncwarp();
-      }
+      const LevelUnit<G, LU> unit = next;
+      next.fetch(cp, ip, rp);
+      unit.run(X, inv_offset, carry);
     }
   }
 
-  // Gathered sums of this warp's items: acc = sum coef * element, in term
-  // order; out(target, flag, acc) takes each sum.  Units as in run_levels.
-  template<int G, class Out>
-  __device__ __forceinline__ void run_gather(const DevGroupPhase& ph, const GroupThread<G>& X, Out out)
+  // One unit of a gather: sums of coef * element, in term order.
+  template<int G>
+  struct GatherUnit
   {
-    constexpr int ipw = 32 / G, U = kGroupUnit;
-    int32_t u = ph.warp_start[X.warp];
-    const int32_t u1 = ph.warp_start[X.warp + 1];
-    if (u == u1)
-      return;
-    const uint4* cp = ph.ctrl + u;
-    const uint4* ip = ph.item + (int64_t)u * ipw + X.sub;
-    const uint4* rp = ph.row + (int64_t)u * (U * ipw) + X.sub;
-    const double2* fp = ph.coef + (int64_t)u * (U * 2 * ipw) + X.sub;
-    uint4 nctrl = __ldg(cp), nitem = __ldg(ip), nrow[U];
-    double2 nf[2 * U];
-#pragma unroll
-    for (int j = 0; j < U; ++j)
+    uint32_t ctrl;
+    uint4 item, row[2];
+    double2 f[8];
+
+    __device__ __forceinline__ void fetch(const uint32_t*& cp, const uint4*& ip, const uint4*& rp, const double2*& fp)
     {
-      nrow[j] = __ldg(rp + j * ipw);
-      nf[2 * j] = __ldg(fp + 2 * j * ipw);
-      nf[2 * j + 1] = __ldg(fp + (2 * j + 1) * ipw);
-    }
-    double acc = 0.0;
-    for (; u < u1; ++u)
-    {
-      const uint32_t ctrl[U] = { nctrl.x, nctrl.y, nctrl.z, nctrl.w };
-      const uint32_t item[U] = { nitem.x, nitem.y, nitem.z, nitem.w };
-      uint4 row[U];
-      double2 f[2 * U];
+      constexpr int ipw = 32 / G;
+      ctrl = __ldg(cp);
+      item = __ldg(ip);
+      row[0] = __ldg(rp);
+      row[1] = __ldg(rp + ipw);
 #pragma unroll
-      for (int j = 0; j < U; ++j)
-      {
-        row[j] = nrow[j];
-        f[2 * j] = nf[2 * j];
-        f[2 * j + 1] = nf[2 * j + 1];
-      }
+      for (int j = 0; j < 8; ++j)
+        f[j] = __ldg(fp + j * ipw);
       cp += 1;
       ip += ipw;
-      rp += U * ipw;
-      fp += U * 2 * ipw;
-      nctrl = __ldg(cp);
-      nitem = __ldg(ip);
+      rp += 2 * ipw;
+      fp += 8 * ipw;
+    }
+
+    template<int C, int T, bool LAST>
+    __device__ __forceinline__ void run(const GroupThread<G>& X, double alpha, double& carry) const
+    {
+      double acc[C];
 #pragma unroll
-      for (int j = 0; j < U; ++j)
-      {
-        nrow[j] = __ldg(rp + j * ipw);
-        nf[2 * j] = __ldg(fp + 2 * j * ipw);
-        nf[2 * j + 1] = __ldg(fp + (2 * j + 1) * ipw);
-      }
+      for (int k = 0; k < C; ++k)
+        acc[k] = 0.0;
+      if (C == 1 && T == 16 && !(ctrl & 1024u))
+        acc[0] = carry;
 #pragma unroll
-      for (int j = 0; j < U; ++j)
+      for (int t = 0; t < T; ++t)
       {
-        const uint32_t c = ctrl[j];
-        if (c & 8u)
-          acc = 0.0;
-        if (c & 7u)
+        double p[C];
+#pragma unroll
+        for (int k = 0; k < C; ++k)
         {
-          const double p0 = f[2 * j].x * X.at(row[j].x), p1 = f[2 * j].y * X.at(row[j].y);
-          const double p2 = f[2 * j + 1].x * X.at(row[j].z), p3 = f[2 * j + 1].y * X.at(row[j].w);
-          acc += p0;
-          acc += p1;
-          acc += p2;
-          acc += p3;
+          const int i = k * (16 / C) + t;
+          const uint4 q = row[i / 8];
+          const uint32_t w = (i / 2) % 4 == 0 ? q.x : ((i / 2) % 4 == 1 ? q.y : ((i / 2) % 4 == 2 ? q.z : q.w));
+          p[k] = (i % 2 ? f[i / 2].y : f[i / 2].x) * X.load(i % 2 ? X.hi(w) : X.lo(w));
         }
-        if ((c & 16u) && item[j] != kGroupNoItem)
-          out(item[j] & 0xFFFFu, item[j] >> 16, acc);
+#pragma unroll
+        for (int k = 0; k < C; ++k)
+          acc[k] += p[k];
       }
+      if (C == 1 && !LAST)
+        carry = acc[0];
+      else
+#pragma unroll
+        for (int k = 0; k < C; ++k)
+        {
+          const uint32_t it = k == 0 ? item.x : (k == 1 ? item.y : (k == 2 ? item.z : item.w));
+          // no sum is -0 (it starts at +0), so adding 0 changes none
+          X.store(X.lo(it), acc[k] + (it >> 16 ? alpha : 0.0));
+        }
+    }
+
+    __device__ __forceinline__ void run(const GroupThread<G>& X, double alpha, double& carry) const
+    {
+      switch (ctrl & 255u)
+      {
+        case 0 * 3: run<1, 4, true>(X, alpha, carry); break;
+        case 1 * 3: run<1, 8, true>(X, alpha, carry); break;
+        case 2 * 3: run<1, 16, true>(X, alpha, carry); break;
+        case 3 * 3: run<2, 4, true>(X, alpha, carry); break;
+        case 4 * 3: run<2, 8, true>(X, alpha, carry); break;
+        case 5 * 3: run<4, 2, true>(X, alpha, carry); break;
+        case 6 * 3: run<4, 4, true>(X, alpha, carry); break;
+        case 2 * 3 + kGroupNone: run<1, 16, false>(X, alpha, carry); break;
+      }
+    }
+  };
+
+  // Gathered sums of this warp's items into their elements; flagged ones gain alpha.
+  template<int G>
+  __device__ __forceinline__ void run_gather(const DevGroupPhase& ph, const GroupThread<G>& X, double alpha)
+  {
+    constexpr int ipw = 32 / G;
+    int32_t u = ph.warp_start[X.warp];
+    const int32_t u1 = ph.warp_start[X.warp + 1];
+    const uint32_t* cp = ph.ctrl + u;
+    const uint4* ip = ph.item + ((int64_t)u * ipw + X.sub);
+    const uint4* rp = ph.row + ((int64_t)u * (2 * ipw) + X.sub);
+    const double2* fp = ph.coef + ((int64_t)u * (8 * ipw) + X.sub);
+    GatherUnit<G> next;
+    double carry = 0.0;
+    if (u < u1)
+      next.fetch(cp, ip, rp, fp);
+#pragma unroll 1
+    for (; u < u1; ++u)
+    {
+      const GatherUnit<G> unit = next;
+      next.fetch(cp, ip, rp, fp);
+      unit.run(X, alpha, carry);
     }
   }
 
@@ -306,15 +409,15 @@ namespace micmb
   // The cells' vectors that stay in global memory (L2), element i at i * G
   struct GroupVectors
   {
-    double *Y, *F0, *Fc, *K;
+    double *Y, *Fc, *K;
     const double* kk;  // rate constants, stride ks
     int32_t ks;
   };
 
-  // doubles of Y, F0, Fc and K per cell
+  // doubles of Y, Fc and K per cell
   __host__ __device__ inline int64_t GroupVectorDoubles(int32_t S, int32_t stages)
   {
-    return (int64_t)S * (3 + stages);
+    return (int64_t)S * (2 + stages);
   }
 
   template<int G>
@@ -323,104 +426,135 @@ namespace micmb
     double* p = slot + (threadIdx.x & (G - 1));
     GroupVectors v;
     v.Y = p;
-    v.F0 = v.Y + (int64_t)P.S * G;
-    v.Fc = v.F0 + (int64_t)P.S * G;
+    v.Fc = v.Y + (int64_t)P.S * G;
     v.K = v.Fc + (int64_t)P.S * G;
     v.kk = nullptr;
     v.ks = 0;
     return v;
   }
 
+  // f(i) for this thread's species, in batches of B whose loads can all be under
+  // way together: load(b, i) fetches (i clamped to the last species), use(b, i)
+  // computes and stores.
+  template<int B, int G, class Load, class Use>
+  __device__ __forceinline__ void for_species_by(const GroupThread<G>& X, int32_t S, Load load, Use use)
+  {
+    for (int32_t i0 = X.lane; i0 < S; i0 += B * X.lanes)
+    {
+#pragma unroll
+      for (int b = 0; b < B; ++b)
+        load(b, min(i0 + b * X.lanes, S - 1));
+#pragma unroll
+      for (int b = 0; b < B; ++b)
+        if (i0 + b * X.lanes < S)
+          use(b, i0 + b * X.lanes);
+    }
+  }
+
+  template<int B, int G, class Load, class Use>
+  __device__ __forceinline__ void for_species(const GroupThread<G>& X, int32_t S, Load load, Use use)
+  {
+    if (S <= 2 * X.lanes)
+      for_species_by<2, G>(X, S, load, use);
+    else
+      for_species_by<B, G>(X, S, load, use);
+  }
+
   // One step attempt of the block's cells from the state in V (and v.Y), step
-  // size H of this thread's cell: forcing (where new_f0), alpha I - J, LU, the
-  // stages.  On return V holds Ynew, v.K the stage vectors, and the elements
-  // P.rate + i the scaled squared errors; the caller synchronises.  The sums
-  // and their order are those of the thread-per-cell routines.
+  // size H of this thread's cell: alpha I - J, LU, then per stage the forcing
+  // (where it is new) and the solve.  On return V holds Ynew, v.K the stage
+  // vectors, and the elements P.rate + i the scaled squared errors; the caller
+  // synchronises.  The sums and their order are those of the thread-per-cell
+  // routines.
   template<int G>
   __device__ __forceinline__ void group_attempt(const DevGroup& P, const DevParams& D, const GroupThread<G>& X,
-                                                const GroupVectors& v, double H, bool new_f0,
-                                                const double* __restrict__ atol, double rtol)
+                                                const GroupVectors& v, double H, const double* __restrict__ atol,
+                                                double rtol)
   {
     const int32_t S = P.S;
-    if (new_f0)
-    {
-      group_rates<G>(P, X, v.kk, v.ks);
-      __syncthreads();
-      run_gather<G>(P.forcing, X, [&](uint32_t i, uint32_t, double acc) { v.F0[i * G] = acc; });
-      __syncthreads();
-    }
     group_drates<G>(P, X, v.kk, v.ks);
     __syncthreads();
-    {
-      const double alpha = 1.0 / (H * D.gamma0);
-      run_gather<G>(P.jacobian, X,
-                    [&](uint32_t e, uint32_t diag, double acc) { X[e] = diag ? acc + alpha : acc; });
-    }
+    run_gather<G>(P.jacobian, X, 1.0 / (H * D.gamma0));
     __syncthreads();
-    run_levels<G>(P.lu, X, P);
-    const double* F = v.F0;
+    if (X.lane == 0)
+      X[P.inv + S] = 1.0;  // the Jacobian rates were there
+    run_levels<G, true>(P.lu, X, P);
     for (int32_t st = 0; st < D.stages; ++st)
     {
       const int32_t sc = st * (st - 1) / 2;
-      double coh[5];
-#pragma unroll
-      for (int32_t j = 0; j < 5; ++j)
-        coh[j] = j < st ? D.c[sc + j] / H : 0.0;
-      // the stage's right-hand side into V
-      auto rhs = [&](uint32_t i, double f) {
-#pragma unroll
-        for (int32_t j = 0; j < 5; ++j)
-          if (j < st)
-            f += coh[j] * v.K[((int64_t)j * S + i) * G];
-        X[P.v0 + i] = f;
-      };
-      if (st > 0 && D.new_f[st])
+      const bool fresh = st == 0 || D.new_f[st];
+      if (fresh)
       {
-#pragma unroll 4
-        for (int32_t i = X.lane; i < S; i += X.lanes)
+        // V holds Y in the first stage
+        if (st > 0)
         {
-          double y = v.Y[(int64_t)i * G];
+          double y[8];
+          for_species<8, G>(
+              X, S,
+              [&](int b, int32_t i) {
+                y[b] = v.Y[(int64_t)i * G];
 #pragma unroll
-          for (int32_t j = 0; j < 5; ++j)
-            if (j < st)
-              y += D.a[sc + j] * v.K[((int64_t)j * S + i) * G];
-          X[P.v0 + i] = y;
+                for (int32_t j = 0; j < 5; ++j)
+                  if (j < st)
+                    y[b] += D.a[sc + j] * v.K[((int64_t)j * S + i) * G];
+              },
+              [&](int b, int32_t i) { X[P.v0 + i] = y[b]; });
+          __syncthreads();
         }
-        __syncthreads();
         group_rates<G>(P, X, v.kk, v.ks);
         __syncthreads();
-        const bool keep = st + 1 < D.stages && !D.new_f[st + 1];
-        run_gather<G>(P.forcing, X, [&](uint32_t i, uint32_t, double acc) {
-          if (keep)
-            v.Fc[i * G] = acc;
-          rhs(i, acc);
-        });
-        F = v.Fc;
+        run_gather<G>(P.forcing, X, 0.0);
+        __syncthreads();
       }
-      else
-        for (int32_t i = X.lane; i < S; i += X.lanes)
-          rhs((uint32_t)i, F[(int64_t)i * G]);
-      __syncthreads();
-      run_levels<G>(P.solve, X, P);
+      // the stage's right-hand side into V
+      const bool keep = fresh && st + 1 < D.stages && !D.new_f[st + 1];
+      if (st > 0 || keep)
+      {
+        double coh[5];
+#pragma unroll
+        for (int32_t j = 0; j < 5; ++j)
+          coh[j] = j < st ? D.c[sc + j] / H : 0.0;
+        double f[8], f0[8];
+        for_species<8, G>(
+            X, S,
+            [&](int b, int32_t i) {
+              f0[b] = f[b] = fresh ? X[P.v0 + i] : v.Fc[(int64_t)i * G];
+#pragma unroll
+              for (int32_t j = 0; j < 5; ++j)
+                if (j < st)
+                  f[b] += coh[j] * v.K[((int64_t)j * S + i) * G];
+            },
+            [&](int b, int32_t i) {
+              if (keep)
+                v.Fc[(int64_t)i * G] = f0[b];
+              X[P.v0 + i] = f[b];
+            });
+        __syncthreads();
+      }
+      run_levels<G, false>(P.solve, X, P);
       __syncthreads();
       for (int32_t i = X.lane; i < S; i += X.lanes)
         v.K[((int64_t)st * S + i) * G] = X[P.v0 + i];
     }
-#pragma unroll 2
-    for (int32_t i = X.lane; i < S; i += X.lanes)
-    {
-      const double y = v.Y[(int64_t)i * G];
-      double yn = y, e = 0.0;
+    double y[4], yn[4], e[4], at[4];
+    for_species<4, G>(
+        X, S,
+        [&](int b, int32_t i) {
+          y[b] = yn[b] = v.Y[(int64_t)i * G];
+          at[b] = atol[i];
+          e[b] = 0.0;
 #pragma unroll
-      for (int32_t st = 0; st < 6; ++st)
-        if (st < D.stages)
-        {
-          const double kv = v.K[((int64_t)st * S + i) * G];
-          yn += D.m[st] * kv;
-          e += D.e[st] * kv;
-        }
-      X[P.v0 + i] = yn;
-      X[P.rate + i] = scaled_sq(y, yn, e, atol[i], rtol);
-    }
+          for (int32_t st = 0; st < 6; ++st)
+            if (st < D.stages)
+            {
+              const double kv = v.K[((int64_t)st * S + i) * G];
+              yn[b] += D.m[st] * kv;
+              e[b] += D.e[st] * kv;
+            }
+        },
+        [&](int b, int32_t i) {
+          X[P.v0 + i] = yn[b];
+          X[P.rate + i] = scaled_sq(y[b], yn[b], e[b], at[b], rtol);
+        });
   }
 }  // namespace micmb

@@ -4,10 +4,12 @@
 //
 // A warp is 32 / G item lanes of G cells each.  The items of a phase (LU
 // entries, solution components, gathered sums) are cut into chunks of 32 / G
-// items, one per item lane; a chunk's terms are stored lane-interleaved and
-// padded to its longest item with products of the zero element, which leave
-// every sum bit-identical.  Every warp walks its own chunk list; the lists of
-// a phase agree on where the block synchronises.
+// items, one per item lane, padded to the chunk's longest sum with products of
+// the zero element, which leave every sum bit-identical.  Chunks are packed into
+// units of 16 terms per lane -- four chunks of up to four terms, two of up to
+// eight, or a stretch of one long chunk -- so that a warp works on independent
+// sums side by side and decides what to do once per unit.  Every warp walks its
+// own list of units; the lists of a phase agree on where the block synchronises.
 #pragma once
 
 #include "mechanism.hpp"
@@ -24,34 +26,38 @@ namespace micmb
     int32_t v0;         // S: the state a rate reads, then the stage vector being solved
     int32_t trash;      // what idle lanes write
     int32_t w0;         // Jacobian rates (n_info), later inv and the rates
-    int32_t inv;        // S: 1 / u_ii
+    int32_t inv;        // S: 1 / u_ii, and 1.0 as the trash element's
     int32_t rate;       // max(R, S): reaction rates, then the scaled squared errors
     int32_t elements;
   };
   GroupLayout MakeGroupLayout(const CompiledMechanism& m);
 
-  constexpr uint32_t kGroupNoItem = 0xFFFFFFFFu;
-  // how a chunk's sums become values
-  constexpr int32_t kGroupScale = 0;  // v * [aux]
-  constexpr int32_t kGroupRecip = 1;  // v, and [aux] = 1 / v
-  constexpr int32_t kGroupDiv = 2;    // v / [aux], with the reciprocal of [aux] at target - v0 + inv
-  constexpr int32_t kGroupStore = 3;  // v
-  // what follows a chunk
+  // What becomes of a unit's sums v.  Level phases: kGroupPlain stores v * [aux] in
+  // the LU and v in the solves; kGroupPivot stores v and [aux] = 1 / v in the LU, and
+  // v / [aux] in the solves (the reciprocal of [aux] is at target - v0 + inv).
+  // kGroupNone: a stretch of a long sum that goes on in the next unit.
+  constexpr int32_t kGroupPlain = 0, kGroupPivot = 1, kGroupNone = 2;
+  // what follows a unit
   constexpr int32_t kGroupNoSync = 0, kGroupWarpSync = 1, kGroupBlockSync = 2;
 
-  // A warp's chunks become a straight run of records of up to four terms, read in
-  // units of four records so that a whole unit is fetched while the one before
-  // it is worked on.  Elements appear as byte offsets (element * G * 8), so that
-  // an operand's address is one addition.  Record r = 4 u + j, item lane p:
-  //   ctrl[r]: T | first << 3 | last << 4 | kind << 5 | sync << 7 (T: the record's
-  //            terms, 0..4; first/last record of a chunk)
-  //   level phases: item[((u * ipw + p) * 4 + j) * 2 ..], target and aux;
-  //                 row[((r * 2 + h) * ipw + p) * 4 ..], terms 2 h and 2 h + 1, two
-  //                 operands each; idle lanes work on the trash element
-  //   gathers: item[(u * ipw + p) * 4 + j], target index | flag << 16 (flag: adds
-  //            alpha) or kGroupNoItem; row[(r * ipw + p) * 4 ..], the four values;
-  //            coef[((r * 2 + h) * ipw + p) * 2 ..], their coefficients
-  constexpr int32_t kGroupUnit = 4;
+  // Unit shapes: chunks and terms per chunk.  A unit has room for 16 terms; those
+  // past a chunk's longest sum are not run.
+  struct GroupShape
+  {
+    int32_t chunks, terms;
+  };
+  constexpr GroupShape kGroupShapes[7] = { { 1, 4 }, { 1, 8 }, { 1, 16 }, { 2, 4 }, { 2, 8 }, { 4, 2 }, { 4, 4 } };
+  constexpr int32_t kGroupTerms = 16;
+
+  // Unit u, item lane p (chunk k starts at term k * 16 / chunks):
+  //   ctrl[u]: shape * 3 + what becomes of the sums | sync << 8 | (first unit of a
+  //            sum) << 10
+  //   item[(u * ipw + p) * 4 + k]: chunk k's target | aux << 16 (gathers: aux 1 adds
+  //            alpha); idle lanes work on the trash element
+  //   the unit's terms t = 0..15 of the lane:
+  //     level phases: row[((u * 4 + t / 4) * ipw + p) * 4 + t % 4], a | b << 16
+  //     gathers: row[((u * 2 + t / 8) * ipw + p) * 4 + t % 8 / 2], the values, two per
+  //              word; coef[((u * 8 + t / 2) * ipw + p) * 2 + t % 2]
   struct GroupPhase
   {
     std::vector<int32_t> warp_start;  // [W + 1] first unit of each warp

@@ -72,7 +72,7 @@ namespace micmb
     // goes to its own array; where the last attempt was accepted, this one reads
     // the state from there and completes it in y.
     template<int G>
-    __global__ void k_global_attempt(DevGroup P, DevParams D, GlobalArgs a, double* ws, int64_t slot_doubles)
+    __global__ void __launch_bounds__(256, 1) k_global_attempt(DevGroup P, DevParams D, GlobalArgs a, double* ws, int64_t slot_doubles)
     {
       extern __shared__ __align__(16) double shared[];
       if (a.ctl->status != MICMB_SOLVER_RUNNING)
@@ -106,7 +106,7 @@ namespace micmb
             a.y[by + (size_t)i * L] = yi;
         }
         __syncthreads();
-        group_attempt<G>(P, D, X, v, H, true, a.atol, a.rtol);
+        group_attempt<G>(P, D, X, v, H, a.atol, a.rtol);
         if (live)
           for (int32_t i = X.lane; i < S; i += X.lanes)
             a.ynew[by + (size_t)i * L] = X[P.v0 + i];
