@@ -25,6 +25,7 @@
 //     a logical AND over all cells and species, so the result is independent
 //     of the cell count's grouping: bit for bit micm's.
 #include "runtime.hpp"
+#include "group.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -141,6 +142,68 @@ namespace micmb
       int32_t st[7];  // function_calls, jacobian_updates, number_of_steps, accepted, rejected, decompositions, solves
     };
 
+    __device__ __forceinline__ void be_start(BeCell& c, const BeParams& P, double dt)
+    {
+      c = BeCell{};
+      c.H = P.h_start == 0.0 ? dt : P.h_start;
+      c.state = MICMB_SOLVER_RUNNING;
+    }
+
+    // what becomes of the cell's state after a Newton iteration
+    constexpr int32_t kBeGoOn = 0;      // iterate again
+    constexpr int32_t kBeAccepted = 1;  // Yn <- Y
+    constexpr int32_t kBeRejected = 2;  // Y <- Yn
+    constexpr int32_t kBeDone = 4;      // and the solve is over
+
+    // micm's decisions after one Newton iteration of one cell
+    __device__ __forceinline__ int32_t be_after_iteration(BeCell& c, const BeParams& P, double dt, bool all_small,
+                                                          bool any_nan, bool any_inf)
+    {
+      c.st[0] += 1;  // function_calls
+      c.st[1] += 1;  // jacobian_updates
+      c.st[2] += 1;  // number_of_steps
+      c.st[5] += 1;  // decompositions
+      c.st[6] += 1;  // solves
+      const bool converged = (c.iterations++ != 0) && all_small;
+      if (!converged && c.iterations < P.max_iter)
+        return kBeGoOn;
+      int32_t what = kBeGoOn;
+      if (!converged)
+      {
+        c.st[4] += 1;
+        c.n_ok = 0;
+        if (c.n_fail >= P.n_red)
+        {
+          c.t = c.t + c.H;
+          c.state = any_nan ? MICMB_SOLVER_NAN_DETECTED
+                            : (any_inf ? MICMB_SOLVER_INF_DETECTED : MICMB_SOLVER_ACCEPTING_UNCONVERGED);
+          return kBeDone;
+        }
+        what = kBeRejected;
+        c.H = c.H * P.red[c.n_fail++];
+      }
+      else
+      {
+        c.st[3] += 1;
+        c.state = MICMB_SOLVER_CONVERGED;
+        c.t = c.t + c.H;
+        what = kBeAccepted;
+        if (++c.n_ok >= 2)
+        {
+          c.n_ok = 0;
+          c.H = c.H * 2.0;
+        }
+      }
+      const double rem = dt - c.t;
+      c.H = (rem < c.H) ? rem : c.H;  // std::min(H, time_step - present_time)
+      c.iterations = 0;
+      if (c.t < dt)
+        c.state = MICMB_SOLVER_RUNNING;
+      else
+        what |= kBeDone;
+      return what;
+    }
+
     __global__ void __launch_bounds__(kThreadsPerBlock, 8)
         k_backward_euler_thread(DevMech M, BeParams P, double dt, FusedArgs A, double* ws, BeLayout T)
     {
@@ -198,9 +261,7 @@ namespace micmb
         }
         for (int32_t r = 0; r < R; ++r)
           kk[r] = A.rate_constants[bk + (size_t)r * L];
-        c = BeCell{};
-        c.H = P.h_start == 0.0 ? dt : P.h_start;
-        c.state = MICMB_SOLVER_RUNNING;
+        be_start(c, P, dt);
         have = true;
       };
 
@@ -209,63 +270,23 @@ namespace micmb
       {
         if (!have)
           continue;
-        c.st[2] += 1;  // number_of_steps
         newton_iteration(M, c.H, Y, Yn, F, LU, inv, kk, scr);
-        c.st[0] += 1;  // function_calls
-        c.st[1] += 1;  // jacobian_updates
-        c.st[5] += 1;  // decompositions
-        c.st[6] += 1;  // solves
-        const bool converged = (c.iterations++ != 0) && cell_converged(M, P, A.atol, A.rtol, F, Y);
-        if (!converged && c.iterations < P.max_iter)
-          continue;
-        bool done = false;
-        if (!converged)
-        {
-          c.st[4] += 1;
-          c.n_ok = 0;
-          if (c.n_fail >= P.n_red)
+        bool any_nan = false, any_inf = false;
+        const bool small = c.iterations != 0 && cell_converged(M, P, A.atol, A.rtol, F, Y);
+        if (!small && c.iterations + 1 >= P.max_iter)
+          for (int32_t i = 0; i < S; ++i)
           {
-            c.t = c.t + c.H;
-            bool any_nan = false, any_inf = false;
-            for (int32_t i = 0; i < S; ++i)
-            {
-              any_nan = any_nan || isnan(Y[i]);
-              any_inf = any_inf || isinf(Y[i]);
-            }
-            c.state = any_nan ? MICMB_SOLVER_NAN_DETECTED
-                              : (any_inf ? MICMB_SOLVER_INF_DETECTED : MICMB_SOLVER_ACCEPTING_UNCONVERGED);
-            done = true;
+            any_nan = any_nan || isnan(Y[i]);
+            any_inf = any_inf || isinf(Y[i]);
           }
-          else
-          {
-            for (int32_t i = 0; i < S; ++i)
-              Y[i] = Yn[i];
-            c.H = c.H * P.red[c.n_fail++];
-          }
-        }
-        else
-        {
-          c.st[3] += 1;
-          c.state = MICMB_SOLVER_CONVERGED;
-          c.t = c.t + c.H;
+        const int32_t what = be_after_iteration(c, P, dt, small, any_nan, any_inf);
+        if (what & kBeAccepted)
           for (int32_t i = 0; i < S; ++i)
             Yn[i] = Y[i];
-          if (++c.n_ok >= 2)
-          {
-            c.n_ok = 0;
-            c.H = c.H * 2.0;
-          }
-        }
-        if (!done)
-        {
-          const double rem = dt - c.t;
-          c.H = (rem < c.H) ? rem : c.H;  // std::min(H, time_step - present_time)
-          c.iterations = 0;
-          if (c.t < dt)
-            c.state = MICMB_SOLVER_RUNNING;
-          else
-            done = true;
-        }
+        if (what & kBeRejected)
+          for (int32_t i = 0; i < S; ++i)
+            Y[i] = Yn[i];
+        const bool done = what & kBeDone;
         if (done)
         {
           write_out();
@@ -273,6 +294,128 @@ namespace micmb
         }
       }
       __syncthreads();
+      if (threadIdx.x < 8 && block_stats[threadIdx.x])
+        atomicAdd(A.stats + threadIdx.x, block_stats[threadIdx.x]);
+    }
+
+    // one value's part of IsConverged (backward_euler.inl:188-246)
+    __device__ __forceinline__ bool value_converged(const BeParams& P, double atol, double rtol, double d, double y)
+    {
+      const double r = fabs(d);
+      return isfinite(d) && !(r > P.small && r > atol && r > rtol * fabs(y));
+    }
+
+    constexpr int32_t kBeBig = 1, kBeNan = 2, kBeInf = 4;  // what an iteration found
+
+    // Per cell on the cell-group engine (group.cuh): a block iterates G cells in
+    // lockstep with their factors in shared memory.  Same decisions and the same
+    // sums as k_backward_euler_thread.
+    template<int G>
+    __global__ void __launch_bounds__(256, 1)
+        k_group_euler(DevGroup P, BeParams B, double dt, FusedArgs A, double* ws, int64_t slot_doubles)
+    {
+      extern __shared__ __align__(16) double shared[];
+      __shared__ BeCell ctl[G];
+      __shared__ int64_t cell_of[G];
+      __shared__ int32_t what[G], found[G];
+      __shared__ unsigned long long block_stats[8];
+      const GroupThread<G> X(shared);
+      const int32_t g = threadIdx.x & (G - 1), S = P.S, L = A.L;
+      double* slot = ws + (int64_t)blockIdx.x * slot_doubles;
+      GroupVectors v = group_vectors<G>(slot, P);
+      double* kk = slot + GroupVectorDoubles(S, 0) * G + g;
+      v.kk = kk;
+      v.ks = G;
+      constexpr int32_t kNew = 8, kIdle = 16;  // beside the outcomes of be_after_iteration
+      if (threadIdx.x < 8)
+        block_stats[threadIdx.x] = 0;
+      if (X.lane == 0)
+      {
+        X[P.zero] = 0.0;
+        X[P.one] = 1.0;
+        X[P.trash] = 1.0;
+        be_start(ctl[g], B, dt);
+      }
+      for (int32_t i = X.lane; i < S; i += X.lanes)
+        X[P.v0 + i] = v.Y[(int64_t)i * G] = v.Fc[(int64_t)i * G] = 0.0;
+      for (int32_t r = X.lane; r < P.R; r += X.lanes)
+        kk[(int64_t)r * G] = 0.0;
+      auto claim = [&]() {
+        const int64_t c = atomicAdd(A.next_cell, 1);
+        const bool have = c < A.n_cells;
+        cell_of[g] = have ? c : -1;
+        what[g] = have ? kNew : kIdle;
+        be_start(ctl[g], B, dt);
+      };
+      if (threadIdx.x < G)
+        claim();
+      for (;;)
+      {
+        __syncthreads();
+        int32_t w = what[g];
+        if (!__syncthreads_or(w != kIdle))
+          break;
+        if (w == kNew)
+        {
+          const double* y = A.variables_in + cell_base(cell_of[g], L, S);
+          const double* k = A.rate_constants + cell_base(cell_of[g], L, P.R);
+          for (int32_t i = X.lane; i < S; i += X.lanes)
+            X[P.v0 + i] = v.Y[(int64_t)i * G] = v.Fc[(int64_t)i * G] = y[(int64_t)i * L];
+          for (int32_t r = X.lane; r < P.R; r += X.lanes)
+            kk[(int64_t)r * G] = k[(int64_t)r * L];
+        }
+        if (X.lane == 0)
+          found[g] = 0;
+        __syncthreads();
+        int32_t bits = 0;
+        group_newton<G>(P, X, v, ctl[g].H, [&](int32_t i, double d, double y) {
+          bits |= (value_converged(B, A.atol[i], A.rtol, d, y) ? 0 : kBeBig) | (isnan(y) ? kBeNan : 0) |
+                  (isinf(y) ? kBeInf : 0);
+        });
+        if (bits)
+          atomicOr(found + g, bits);
+        __syncthreads();
+        if (threadIdx.x < G && w != kIdle)
+        {
+          BeCell c = ctl[g];
+          what[g] = be_after_iteration(c, B, dt, !(found[g] & kBeBig), found[g] & kBeNan, found[g] & kBeInf);
+          ctl[g] = c;
+        }
+        __syncthreads();
+        w = what[g];
+        if (w != kIdle)
+        {
+          if (w & kBeAccepted)
+            for (int32_t i = X.lane; i < S; i += X.lanes)
+              v.Fc[(int64_t)i * G] = X[P.v0 + i];
+          if (w & kBeRejected)
+            for (int32_t i = X.lane; i < S; i += X.lanes)
+              X[P.v0 + i] = v.Y[(int64_t)i * G] = v.Fc[(int64_t)i * G];
+          if (w & kBeDone)
+          {
+            double* out = A.variables_out + cell_base(cell_of[g], L, S);
+            for (int32_t i = X.lane; i < S; i += X.lanes)
+            {
+              const double y = X[P.v0 + i];
+              out[(int64_t)i * L] = (y < 0.0) ? 0.0 : y;
+            }
+          }
+        }
+        __syncthreads();
+        if (threadIdx.x < G && w != kIdle && (w & kBeDone))
+        {
+          const BeCell& c = ctl[g];
+          if (A.cell_status)
+            A.cell_status[cell_of[g]] = c.state;
+          if (A.cell_accepted)
+            A.cell_accepted[cell_of[g]] = c.st[3];
+          for (int q = 0; q < 7; ++q)
+            atomicAdd(block_stats + q, (unsigned long long)c.st[q]);
+          if (c.state != MICMB_SOLVER_CONVERGED)
+            atomicAdd(block_stats + 7, 1ull);
+          claim();
+        }
+      }
       if (threadIdx.x < 8 && block_stats[threadIdx.x])
         atomicAdd(A.stats + threadIdx.x, block_stats[threadIdx.x]);
     }
@@ -348,6 +491,109 @@ namespace micmb
         atomicOr(&w->any_nan, 1);
       if (any_inf)
         atomicOr(&w->any_inf, 1);
+    }
+
+    // k_be_iterate on the cell-group engine: one Newton iteration of every cell, a
+    // block taking the cells group by group.
+    template<int G>
+    __global__ void __launch_bounds__(256, 1)
+        k_group_be_iterate(DevGroup P, BeParams B, BeArgs a, double* ws, int64_t slot_doubles)
+    {
+      extern __shared__ __align__(16) double shared[];
+      BeCtl* ctl = a.ctl;
+      if (ctl->phase != 0)
+        return;
+      const GroupThread<G> X(shared);
+      const int32_t S = P.S, L = a.L;
+      GroupVectors v = group_vectors<G>(ws + (int64_t)blockIdx.x * slot_doubles, P);
+      v.ks = L;
+      const double H = ctl->H;
+      const bool check = ctl->iterations != 0;
+      if (X.lane == 0)
+      {
+        X[P.zero] = 0.0;
+        X[P.one] = 1.0;
+        X[P.trash] = 1.0;
+      }
+      int32_t bits = 0;
+      for (int64_t first = (int64_t)blockIdx.x * G; first < a.n; first += (int64_t)gridDim.x * G)
+      {
+        const int64_t c = first + (threadIdx.x & (G - 1));
+        const bool live = c < a.n;
+        const int64_t cc = live ? c : a.n - 1;
+        double* y = a.y + cell_base(cc, L, S);
+        const double* yn = a.yn + cell_base(cc, L, S);
+        v.kk = a.k + cell_base(cc, L, P.R);
+        for (int32_t i = X.lane; i < S; i += X.lanes)
+        {
+          X[P.v0 + i] = v.Y[(int64_t)i * G] = live ? y[(int64_t)i * L] : 0.0;
+          v.Fc[(int64_t)i * G] = live ? yn[(int64_t)i * L] : 0.0;
+        }
+        __syncthreads();
+        group_newton<G>(P, X, v, H, [&](int32_t i, double d, double yi) {
+          if (live)
+          {
+            y[(int64_t)i * L] = yi;
+            bits |= (check && !value_converged(B, a.atol[i], a.rtol, d, yi) ? kBeBig : 0) |
+                    (isnan(yi) ? kBeNan : 0) | (isinf(yi) ? kBeInf : 0);
+          }
+        });
+        __syncthreads();
+      }
+      if (bits & kBeBig)
+        atomicOr(&ctl->not_converged, 1);
+      if (bits & kBeNan)
+        atomicOr(&ctl->any_nan, 1);
+      if (bits & kBeInf)
+        atomicOr(&ctl->any_inf, 1);
+    }
+
+    using GroupEulerKernel = void (*)(DevGroup, BeParams, double, FusedArgs, double*, int64_t);
+    using GroupIterateKernel = void (*)(DevGroup, BeParams, BeArgs, double*, int64_t);
+
+    GroupEulerKernel GroupEulerFor(int32_t G)
+    {
+      switch (G)
+      {
+        case 1: return k_group_euler<1>;
+        case 2: return k_group_euler<2>;
+        case 4: return k_group_euler<4>;
+        case 8: return k_group_euler<8>;
+        case 16: return k_group_euler<16>;
+        default: return k_group_euler<32>;
+      }
+    }
+
+    GroupIterateKernel GroupIterateFor(int32_t G)
+    {
+      switch (G)
+      {
+        case 1: return k_group_be_iterate<1>;
+        case 2: return k_group_be_iterate<2>;
+        case 4: return k_group_be_iterate<4>;
+        case 8: return k_group_be_iterate<8>;
+        case 16: return k_group_be_iterate<16>;
+        default: return k_group_be_iterate<32>;
+      }
+    }
+
+    // blocks of a cell-group kernel for n cells and the vectors of each; 0 blocks:
+    // the mechanism does not fit
+    struct GroupGrid
+    {
+      int64_t blocks = 0, slot = 0;
+    };
+
+    GroupGrid PrepareGroup(micmb_solver& s, micmb_state& st, const void* kernel, const GroupChoice& choice, int64_t n,
+                           int64_t doubles_per_cell)
+    {
+      GroupGrid gg;
+      const int per_sm = GroupBlocksPerSm(s, kernel, choice);
+      gg.blocks = std::min<int64_t>((int64_t)per_sm * s.sm_count, (n + choice.G - 1) / choice.G);
+      gg.slot = doubles_per_cell * choice.G;
+      if (gg.blocks > 0 && st.group_ws.bytes < sizeof(double) * (size_t)(gg.blocks * gg.slot))
+        st.group_ws = DeviceMemory(sizeof(double) * (size_t)(gg.blocks * gg.slot));
+      return gg;
     }
 
     // micm's decisions after one Newton iteration (backward_euler.inl:55-179)
@@ -471,9 +717,21 @@ namespace micmb
     void SolveBackwardEulerGlobal(micmb_solver& s, micmb_state& st, double dt, const BeParams& P,
                                   micmb_solver_stats* stats, int32_t* per_cell_status, int32_t* per_cell_accepted)
     {
-      EnsurePlainBuffers(st);
       const auto& m = *s.mech;
       const int64_t n = st.n_cells;
+      const bool group = n > 0 && GroupVariantApplies(s, n);
+      const GroupChoice choice = group ? ChooseGroup(s, n) : GroupChoice{ 1, 1 };
+      const GroupIterateKernel iterate = GroupIterateFor(choice.G);
+      const DevGroup tables = group ? GroupTablesFor(s, choice).dev : DevGroup{};
+      GroupGrid gg;
+      if (group)
+      {
+        gg = PrepareGroup(s, st, reinterpret_cast<const void*>(iterate), choice, n, GroupVectorDoubles(m.S, 0));
+        if (!st.group_ynew.p)
+          st.group_ynew = DeviceMemory(st.dense_bytes(m.S));
+      }
+      else
+        EnsurePlainBuffers(st);
       if (!st.be_ctl.p)
         st.be_ctl = DeviceMemory(sizeof(BeCtl));
       BeArgs a{};
@@ -481,7 +739,7 @@ namespace micmb
       a.L = st.L;
       a.scratch_cols = std::max<int32_t>(m.R, (int32_t)m.info_rxn.size());
       a.y = st.variables.as<double>();
-      a.yn = st.ynew.as<double>();
+      a.yn = (group ? st.group_ynew : st.ynew).as<double>();
       a.f = st.forcing0.as<double>();
       a.jac = st.jacobian.as<double>();
       a.inv = st.inv_diag.as<double>();
@@ -508,7 +766,11 @@ namespace micmb
         {
           for (int64_t it = 0; it < batch; ++it)
           {
-            k_be_iterate<<<grid_c, kBlock, 0, stream>>>(s.dev, P, a);
+            if (group)
+              iterate<<<(unsigned)gg.blocks, 32 * choice.W, GroupSharedBytes(s, choice), stream>>>(
+                  tables, P, a, st.group_ws.as<double>(), gg.slot);
+            else
+              k_be_iterate<<<grid_c, kBlock, 0, stream>>>(s.dev, P, a);
             k_be_control<<<1, 1, 0, stream>>>(P, dt, a.ctl);
             k_be_apply<<<grid_e, kBlock, 0, stream>>>(a, S);
           }
@@ -565,16 +827,7 @@ namespace micmb
     {
       const auto& m = *s.mech;
       const int64_t n = st.n_cells;
-      const BeLayout T = MakeBeLayout(m.S, m.R, (int32_t)m.info_rxn.size(), m.nnz);
-      int per_sm = 0;
-      MICMB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_backward_euler_thread, kThreadsPerBlock, 0));
-      if (per_sm < 1)
-        throw Error(MICMB_ERR_UNSUPPORTED, "Backward Euler kernel cannot be resident");
-      int64_t grid = (int64_t)per_sm * s.sm_count;
-      grid = std::max<int64_t>(1, std::min<int64_t>(grid, (n + kThreadsPerBlock - 1) / kThreadsPerBlock));
-      const int64_t doubles = grid * kThreadsPerBlock * (int64_t)T.per_slot;
-      if (!st.thread_ws.p || st.thread_ws.bytes < (size_t)doubles * sizeof(double))
-        st.thread_ws = DeviceMemory((size_t)doubles * sizeof(double));
+      const bool group = n > 0 && GroupVariantApplies(s, n);
       if (!st.status.p)
         st.status = DeviceMemory(sizeof(int32_t) * std::max<int64_t>(n, 1));
       if (!st.accepted.p)
@@ -594,8 +847,28 @@ namespace micmb
       A.cell_accepted = st.accepted.as<int32_t>();
       cudaStream_t stream = st.stream;
       MICMB_CUDA(cudaMemsetAsync(cbase, 0, 128, stream));
-      if (n > 0)
+      if (group)
       {
+        const GroupChoice choice = ChooseGroup(s, n);
+        const GroupEulerKernel kernel = GroupEulerFor(choice.G);
+        const GroupGrid gg = PrepareGroup(s, st, reinterpret_cast<const void*>(kernel), choice, n,
+                                          GroupVectorDoubles(m.S, 0) + m.R);
+        kernel<<<(unsigned)gg.blocks, 32 * choice.W, GroupSharedBytes(s, choice), stream>>>(
+            GroupTablesFor(s, choice).dev, P, dt, A, st.group_ws.as<double>(), gg.slot);
+        MICMB_CUDA(cudaGetLastError());
+      }
+      else if (n > 0)
+      {
+        const BeLayout T = MakeBeLayout(m.S, m.R, (int32_t)m.info_rxn.size(), m.nnz);
+        int per_sm = 0;
+        MICMB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_backward_euler_thread, kThreadsPerBlock, 0));
+        if (per_sm < 1)
+          throw Error(MICMB_ERR_UNSUPPORTED, "Backward Euler kernel cannot be resident");
+        int64_t grid = (int64_t)per_sm * s.sm_count;
+        grid = std::max<int64_t>(1, std::min<int64_t>(grid, (n + kThreadsPerBlock - 1) / kThreadsPerBlock));
+        const int64_t doubles = grid * kThreadsPerBlock * (int64_t)T.per_slot;
+        if (!st.thread_ws.p || st.thread_ws.bytes < (size_t)doubles * sizeof(double))
+          st.thread_ws = DeviceMemory((size_t)doubles * sizeof(double));
         k_backward_euler_thread<<<(unsigned)grid, kThreadsPerBlock, 0, stream>>>(s.dev, P, dt, A,
                                                                                   st.thread_ws.as<double>(), T);
         MICMB_CUDA(cudaGetLastError());

@@ -557,4 +557,45 @@ namespace micmb
           X[P.rate + i] = scaled_sq(y[b], yn[b], e[b], at[b], rtol);
         });
   }
+
+  // One Newton iteration of Backward Euler on the block's cells (backward_euler.cu:
+  // newton_iteration) from the state in V and v.Y, with the step's start in v.Fc:
+  // Y <- max(0, Y + (LU)^-1 (f(Y) - (Y - Yn) / H)), into V and v.Y.  test(i, d, y)
+  // sees every correction and new value.
+  template<int G, class Test>
+  __device__ __forceinline__ void group_newton(const DevGroup& P, const GroupThread<G>& X, const GroupVectors& v,
+                                               double H, Test test)
+  {
+    const int32_t S = P.S;
+    group_drates<G>(P, X, v.kk, v.ks);
+    __syncthreads();
+    run_gather<G>(P.jacobian, X, 1.0 / H);
+    __syncthreads();
+    if (X.lane == 0)
+      X[P.inv + S] = 1.0;  // the Jacobian rates were there
+    run_levels<G, true>(P.lu, X, P);
+    group_rates<G>(P, X, v.kk, v.ks);
+    __syncthreads();
+    run_gather<G>(P.forcing, X, 0.0);
+    __syncthreads();
+    double y[4], yn[4];
+    for_species<4, G>(
+        X, S,
+        [&](int b, int32_t i) {
+          y[b] = v.Y[(int64_t)i * G];
+          yn[b] = v.Fc[(int64_t)i * G];
+        },
+        [&](int b, int32_t i) { X[P.v0 + i] = X[P.v0 + i] - (y[b] - yn[b]) / H; });
+    __syncthreads();
+    run_levels<G, false>(P.solve, X, P);
+    __syncthreads();
+    for_species<4, G>(
+        X, S, [&](int b, int32_t i) { y[b] = v.Y[(int64_t)i * G]; },
+        [&](int b, int32_t i) {
+          const double d = X[P.v0 + i], sum = y[b] + d, yi = (0.0 > sum) ? 0.0 : sum;
+          v.Y[(int64_t)i * G] = yi;
+          X[P.v0 + i] = yi;
+          test(i, d, yi);
+        });
+  }
 }  // namespace micmb

@@ -77,3 +77,30 @@ def test_one_cell_global_equals_per_cell(cuda_device):
     y_g, r_g = _solve(Solver(mech, 4, vector_length=8), inp, dt, "plain", "global")
     np.testing.assert_array_equal(y_g, y_p)
     assert r_g.stats["accepted"] == r_p.stats["accepted"] and r_g.stats["rejected"] == r_p.stats["rejected"]
+
+
+@pytest.mark.parametrize("name,n", [("readme", 10007), ("c60", 1201), ("c210", 299)])
+@pytest.mark.parametrize("control", ["per_cell", "global"])
+def test_backward_euler_does_not_depend_on_the_block_shape(cuda_device, name, n, control):
+    """Cells solved together (several per block) equal the same cells in states
+    small enough for one per block; globally, a state of equal cells."""
+    make, inputs, dt = CASES[name]
+    mech = make()
+    inp = inputs(mech, n)
+    if control == "global":  # the step sequence is then each cell's own
+        inp = {k: np.repeat(v[:1], n, axis=0) for k, v in inp.items()}
+
+    def solve(cells):
+        solver = Solver(mech, 3, vector_length=32)
+        st = make_state(solver, {k: np.ascontiguousarray(v[cells]) for k, v in inp.items()})
+        solver.update_state_parameters(st)
+        res = solver.solve_backward_euler(dt, st, step_control=control, per_cell=True)
+        st.sync_outputs_to_host()
+        return st.concentrations(), res
+
+    y, r = solve(slice(0, n))
+    for cells in (slice(0, 1), slice(n - 100, n)):
+        y_few, r_few = solve(cells)
+        np.testing.assert_array_equal(y[cells], y_few)
+        np.testing.assert_array_equal(r.per_cell_status[cells], r_few.per_cell_status)
+        np.testing.assert_array_equal(r.per_cell_accepted[cells], r_few.per_cell_accepted)
