@@ -168,7 +168,10 @@ extern "C"
         const bool has_stream = solver->dev.has_warp && solver->stream_blocks.p;
         for (const auto& c : candidates)
         {
-          if ((c.variant == 0 && !has_stream) || (c.variant == 1 && !solver->dev.has_warp))
+          const bool group = c.variant == 0 && GroupVariantApplies(*solver, trial_cells(c));
+          // the cell-group kernel takes none of the streamed kernel's settings: one trial
+          if ((c.variant == 0 && !(group ? &c == candidates : has_stream)) ||
+              (c.variant == 1 && !solver->dev.has_warp))
             continue;
           const double r = rate_of(c, trial_cells(c), 2);
           if (r > rate_of_best[c.variant])

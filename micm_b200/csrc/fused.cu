@@ -361,7 +361,10 @@ namespace micmb
     const int64_t n = (adj && adj->n_cells > 0)
                           ? adj->n_cells
                           : (st.solve_limit > 0 ? std::min<int64_t>(st.solve_limit, st.n_cells) : st.n_cells);
-    if (n > 0 && s.fused.variant == 0 && GroupVariantApplies(s, n))
+    // variant 2 without a chosen build: the thread kernel where it is the faster one
+    const bool group = n > 0 && ((s.fused.variant == 0 && GroupVariantApplies(s, n)) ||
+                                 (s.fused.variant == 2 && s.fused.ctas_per_sm == 0 && GroupFaster(s, n)));
+    if (group)
     {
       const FusedArgs A = PerCellArgs(st, adj, n);
       SolveFusedGroup(s, st, A, dt);
@@ -434,7 +437,7 @@ namespace micmb
   bool SolvePlainPerCellGroup(micmb_solver& s, micmb_state& st, double dt, micmb_solver_stats* stats,
                               int32_t* per_cell_status, int32_t* per_cell_accepted)
   {
-    if (st.n_cells < 1 || !GroupVariantApplies(s, st.n_cells))
+    if (st.n_cells < 1 || !GroupFasterThanStages(s, st.n_cells))
       return false;
     const FusedArgs A = PerCellArgs(st, nullptr, st.n_cells);
     SolveFusedGroup(s, st, A, dt);

@@ -362,6 +362,36 @@ namespace micmb
     return GroupBlocksPerSm(s, reinterpret_cast<const void*>(SolveKernelFor(choice.G)), choice) > 0;
   }
 
+  // The thread-per-cell kernels need about 300,000 cells to fill the GPU and take
+  // nearly the same time for fewer; the cell-group kernel's time is proportional
+  // to the cells from a few thousand on, and inversely to the cells an SM holds.
+  // Measured, cell-group against one-cell-per-thread fused kernel, ms: Chapman
+  // 100,000 cells 1.9 / 2.2, 1,000,000 19 / 16; 60 species 262,144 411 / 526,
+  // 1,000,000 1,550 / 1,218; TS1 200,000 1,169 / 1,413, 1,000,000 5,806 / 4,531; 210
+  // species (8 cells per SM) 131,072 933 / 1,478, 262,144 1,859 / 1,896, 524,288
+  // 3,710 / 3,340; 600 species (2 per SM) 20,000 2,532 / 6,182, 100,000 12,593 / 7,442.
+  bool GroupFaster(const micmb_solver& s, int64_t n_cells)
+  {
+    if (!GroupVariantApplies(s, n_cells))
+      return false;
+    return n_cells <= std::min<int64_t>((int64_t)s.sm_count * 2048, 32768 * (int64_t)GroupCellsPerSm(s));
+  }
+
+  // The per-stage kernels take 1.3-1.6 times the thread kernel's time, so with
+  // eight cells per SM the cell-group kernel is faster at any count (210 species,
+  // 1,048,576 cells: 7.4 s against 8.7 s); with two (600 species) it is up to the
+  // thread kernel's limit.
+  bool GroupFasterThanStages(const micmb_solver& s, int64_t n_cells)
+  {
+    return GroupVariantApplies(s, n_cells) && (GroupCellsPerSm(s) >= 8 || GroupFaster(s, n_cells));
+  }
+
+  int32_t GroupCellsPerSm(const micmb_solver& s)
+  {
+    const GroupChoice most = ChooseGroup(s, (int64_t)1 << 40);
+    return most.G * GroupBlocksPerSm(s, reinterpret_cast<const void*>(SolveKernelFor(most.G)), most);
+  }
+
   void SolveFusedGroup(micmb_solver& s, micmb_state& st, const FusedArgs& A, double dt)
   {
     const GroupChoice choice = ChooseGroup(s, A.n_cells);

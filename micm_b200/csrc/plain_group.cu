@@ -256,7 +256,7 @@ namespace micmb
   {
     const auto& m = *s.mech;
     const int64_t n = st.n_cells;
-    if (n < 1 || !GroupApplies(m))
+    if (n < 1 || !GroupFasterThanStages(s, n))
       return false;
     const GroupChoice choice = ChooseGroup(s, n);
     const size_t smem = GroupSharedBytes(s, choice);

@@ -240,6 +240,9 @@ namespace micmb
   size_t GroupSharedBytes(const micmb_solver& s, const GroupChoice& choice);
   int GroupBlocksPerSm(const micmb_solver& s, const void* kernel, const GroupChoice& choice);
   bool GroupVariantApplies(const micmb_solver& s, int64_t n_cells);
+  int32_t GroupCellsPerSm(const micmb_solver& s);
+  bool GroupFaster(const micmb_solver& s, int64_t n_cells);  // than the one-cell-per-thread kernel
+  bool GroupFasterThanStages(const micmb_solver& s, int64_t n_cells);  // than the plain per-stage kernels
   void SolveFusedGroup(micmb_solver& s, micmb_state& st, const FusedArgs& A, double dt);
   // the plain method on them: per cell, or one step size for all cells; false: not taken
   bool SolvePlainPerCellGroup(micmb_solver& s, micmb_state& st, double dt, micmb_solver_stats* stats,
