@@ -161,7 +161,7 @@ namespace micmb
           const int32_t i = st.t0 + t % per_chunk;
           const bool real = u && i < (int32_t)u->term.size();
           if (coef)
-            *coef = real ? u->coef[i] : 0.0;
+            *coef = real ? u->coef[i] : -0.0;  // -0 times the zero element changes no sum, -0 among them
           const uint32_t zero = (uint32_t)L.zero;
           return real ? u->term[i] : (gather ? zero : zero | zero << 16);
         };

@@ -263,13 +263,14 @@ namespace micmb
       fp += 8 * ipw;
     }
 
-    template<int C, int T, bool LAST>
+    // ADD: the sums start from their elements' values, and nothing gains alpha
+    template<bool ADD, int C, int T, bool LAST>
     __device__ __forceinline__ void run(const GroupThread<G>& X, double alpha, double& carry) const
     {
       double acc[C];
 #pragma unroll
       for (int k = 0; k < C; ++k)
-        acc[k] = 0.0;
+        acc[k] = ADD ? X.load(X.lo(k == 0 ? item.x : (k == 1 ? item.y : (k == 2 ? item.z : item.w)))) : 0.0;
       if (C == 1 && T == 16 && !(ctrl & 1024u))
         acc[0] = carry;
 #pragma unroll
@@ -295,29 +296,31 @@ namespace micmb
         for (int k = 0; k < C; ++k)
         {
           const uint32_t it = k == 0 ? item.x : (k == 1 ? item.y : (k == 2 ? item.z : item.w));
-          // no sum is -0 (it starts at +0), so adding 0 changes none
-          X.store(X.lo(it), acc[k] + (it >> 16 ? alpha : 0.0));
+          // a sum that starts at +0 is never -0, so adding 0 changes none
+          X.store(X.lo(it), ADD ? acc[k] : acc[k] + (it >> 16 ? alpha : 0.0));
         }
     }
 
+    template<bool ADD>
     __device__ __forceinline__ void run(const GroupThread<G>& X, double alpha, double& carry) const
     {
       switch (ctrl & 255u)
       {
-        case 0 * 3: run<1, 4, true>(X, alpha, carry); break;
-        case 1 * 3: run<1, 8, true>(X, alpha, carry); break;
-        case 2 * 3: run<1, 16, true>(X, alpha, carry); break;
-        case 3 * 3: run<2, 4, true>(X, alpha, carry); break;
-        case 4 * 3: run<2, 8, true>(X, alpha, carry); break;
-        case 5 * 3: run<4, 2, true>(X, alpha, carry); break;
-        case 6 * 3: run<4, 4, true>(X, alpha, carry); break;
-        case 2 * 3 + kGroupNone: run<1, 16, false>(X, alpha, carry); break;
+        case 0 * 3: run<ADD, 1, 4, true>(X, alpha, carry); break;
+        case 1 * 3: run<ADD, 1, 8, true>(X, alpha, carry); break;
+        case 2 * 3: run<ADD, 1, 16, true>(X, alpha, carry); break;
+        case 3 * 3: run<ADD, 2, 4, true>(X, alpha, carry); break;
+        case 4 * 3: run<ADD, 2, 8, true>(X, alpha, carry); break;
+        case 5 * 3: run<ADD, 4, 2, true>(X, alpha, carry); break;
+        case 6 * 3: run<ADD, 4, 4, true>(X, alpha, carry); break;
+        case 2 * 3 + kGroupNone: run<ADD, 1, 16, false>(X, alpha, carry); break;
       }
     }
   };
 
-  // Gathered sums of this warp's items into their elements; flagged ones gain alpha.
-  template<int G>
+  // Gathered sums of this warp's items into their elements (ADD: added to them);
+  // flagged ones gain alpha.
+  template<int G, bool ADD = false>
   __device__ __forceinline__ void run_gather(const DevGroupPhase& ph, const GroupThread<G>& X, double alpha)
   {
     constexpr int ipw = 32 / G;
@@ -336,7 +339,7 @@ namespace micmb
     {
       const GatherUnit<G> unit = next;
       next.fetch(cp, ip, rp, fp);
-      unit.run(X, alpha, carry);
+      unit.template run<ADD>(X, alpha, carry);
     }
   }
 

@@ -964,15 +964,19 @@ namespace micmb
       }
     }
 
+    // one thread per (cell, species): a thread per cell made 210 dependent round
+    // trips to memory (66 us for 16,384 cells)
     __global__ void k_alpha_minus_jacobian(DevMech M, PlainArgs a, double alpha)
     {
-      const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+      const int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+      const int64_t per_group = (int64_t)M.S * a.L;
+      const int64_t g = idx / per_group;
+      const int32_t rem = (int32_t)(idx - g * per_group);
+      const int64_t c = g * a.L + rem % a.L;
       if (c >= a.n)
         return;
-      const int32_t L = a.L;
-      Strided J{ a.jac + cell_base(c, L, M.nnz), L };
-      for (int32_t i = 0; i < M.S; ++i)
-        J[M.diag_pos[i]] = J[M.diag_pos[i]] + alpha;
+      double& d = a.jac[cell_base(c, a.L, M.nnz) + (size_t)M.diag_pos[rem / a.L] * a.L];
+      d = d + alpha;
     }
 
     __global__ void k_decompose_all(DevMech M, PlainArgs a)
@@ -1016,6 +1020,8 @@ namespace micmb
   void LaunchAddForcing(micmb_solver& s, micmb_state& st)
   {
     EnsurePlainBuffers(st);
+    if (LaunchGroupStage(s, st, GroupStage::kForcing))
+      return;
     PlainArgs a = MakeArgs(s, st, 0);
     k_add_forcing<<<Blocks(st.n_cells), kBlock, 0, st.stream>>>(s.dev, a);
     MICMB_CUDA(cudaGetLastError());
@@ -1023,6 +1029,8 @@ namespace micmb
   void LaunchSubtractJacobian(micmb_solver& s, micmb_state& st)
   {
     EnsurePlainBuffers(st);
+    if (LaunchGroupStage(s, st, GroupStage::kJacobian))
+      return;
     PlainArgs a = MakeArgs(s, st, 0);
     k_subtract_jacobian<<<Blocks(st.n_cells), kBlock, 0, st.stream>>>(s.dev, a);
     MICMB_CUDA(cudaGetLastError());
@@ -1031,12 +1039,14 @@ namespace micmb
   {
     EnsurePlainBuffers(st);
     PlainArgs a = MakeArgs(s, st, 0);
-    k_alpha_minus_jacobian<<<Blocks(st.n_cells), kBlock, 0, st.stream>>>(s.dev, a, alpha);
+    k_alpha_minus_jacobian<<<Blocks(st.n_pad * s.mech->S), kBlock, 0, st.stream>>>(s.dev, a, alpha);
     MICMB_CUDA(cudaGetLastError());
   }
   void LaunchDecompose(micmb_solver& s, micmb_state& st)
   {
     EnsurePlainBuffers(st);
+    if (LaunchGroupStage(s, st, GroupStage::kLu))
+      return;
     PlainArgs a = MakeArgs(s, st, 0);
     k_decompose_all<<<Blocks(st.n_cells), kBlock, 0, st.stream>>>(s.dev, a);
     MICMB_CUDA(cudaGetLastError());
@@ -1044,6 +1054,8 @@ namespace micmb
   void LaunchLinearSolve(micmb_solver& s, micmb_state& st)
   {
     EnsurePlainBuffers(st);
+    if (LaunchGroupStage(s, st, GroupStage::kSolve))
+      return;
     PlainArgs a = MakeArgs(s, st, 0);
     k_linear_solve_all<<<Blocks(st.n_cells), kBlock, 0, st.stream>>>(s.dev, a);
     MICMB_CUDA(cudaGetLastError());

@@ -244,6 +244,15 @@ namespace micmb
   bool GroupFaster(const micmb_solver& s, int64_t n_cells);  // than the one-cell-per-thread kernel
   bool GroupFasterThanStages(const micmb_solver& s, int64_t n_cells);  // than the plain per-stage kernels
   void SolveFusedGroup(micmb_solver& s, micmb_state& st, const FusedArgs& A, double dt);
+  // one stage of every cell (the single-stage entry points); false: not taken
+  enum class GroupStage
+  {
+    kForcing,
+    kJacobian,
+    kLu,
+    kSolve
+  };
+  bool LaunchGroupStage(micmb_solver& s, micmb_state& st, GroupStage stage);
   // the plain method on them: per cell, or one step size for all cells; false: not taken
   bool SolvePlainPerCellGroup(micmb_solver& s, micmb_state& st, double dt, micmb_solver_stats* stats,
                               int32_t* per_cell_status, int32_t* per_cell_accepted);

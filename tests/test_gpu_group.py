@@ -8,7 +8,9 @@ import numpy as np
 import pytest
 
 from micm_b200 import Solver, micm_bench, synthetic
-from gpu_helpers import make_state
+from micm_b200 import solver as sv
+from micm_b200._native import check, lib
+from gpu_helpers import download_cols, make_state, upload_cols
 
 pytestmark = pytest.mark.gpu
 
@@ -104,3 +106,42 @@ def test_backward_euler_does_not_depend_on_the_block_shape(cuda_device, name, n,
         np.testing.assert_array_equal(y[cells], y_few)
         np.testing.assert_array_equal(r.per_cell_status[cells], r_few.per_cell_status)
         np.testing.assert_array_equal(r.per_cell_accepted[cells], r_few.per_cell_accepted)
+
+
+@pytest.mark.parametrize("name,n,L", [("readme", 10007, 32), ("c60", 149, 7), ("c60", 1201, 32), ("c210", 299, 128)])
+def test_single_stages_do_not_depend_on_the_block_shape(cuda_device, name, n, L):
+    """The single-stage entry points on many cells (several per block) equal the
+    same cells in a state small enough for one per block, signed zeros of the
+    accumulated-into arrays included; values outside the real cells stay."""
+    make, inputs, _ = CASES[name]
+    mech = make()
+    inp = inputs(mech, n)
+    S = mech.n_species
+    rng = np.random.default_rng(9)
+    f0 = rng.choice([0.0, -0.0, 1.0e-7], size=(n, S))
+
+    def stages(cells):
+        solver = Solver(mech, 3, vector_length=L)
+        nnz = solver.compiled.info["jacobian_nnz"]
+        j0 = np.random.default_rng(10).choice([0.0, -0.0, 2.0e-3], size=(n, nnz))[cells]
+        st = make_state(solver, {k: np.ascontiguousarray(v[cells]) for k, v in inp.items()})
+        solver.update_state_parameters(st)
+        upload_cols(st, sv.BUF_FORCING, f0[cells])
+        upload_cols(st, sv.BUF_JACOBIAN, j0)
+        out = []
+        check(lib().micmb_add_forcing_terms(solver.handle, st.handle))
+        out.append(download_cols(st, sv.BUF_FORCING, S))
+        check(lib().micmb_subtract_jacobian_terms(solver.handle, st.handle))
+        out.append(download_cols(st, sv.BUF_JACOBIAN, nnz))
+        check(lib().micmb_alpha_minus_jacobian(solver.handle, st.handle, 0.25))
+        out.append(download_cols(st, sv.BUF_JACOBIAN, nnz))
+        check(lib().micmb_lu_decompose(solver.handle, st.handle))
+        out.append(download_cols(st, sv.BUF_JACOBIAN, nnz))
+        check(lib().micmb_linear_solve(solver.handle, st.handle))
+        out.append(download_cols(st, sv.BUF_FORCING, S))
+        return out
+
+    many = stages(slice(0, n))
+    few = stages(slice(n - 100, n))
+    for a, b in zip(many, few):
+        np.testing.assert_array_equal(a[n - 100:].view(np.int64), np.ascontiguousarray(b).view(np.int64))
