@@ -435,11 +435,12 @@ namespace micmb
   }
 
   bool SolvePlainPerCellGroup(micmb_solver& s, micmb_state& st, double dt, micmb_solver_stats* stats,
-                              int32_t* per_cell_status, int32_t* per_cell_accepted)
+                              int32_t* per_cell_status, int32_t* per_cell_accepted, double* cell_time)
   {
     if (st.n_cells < 1 || !GroupFasterThanStages(s, st.n_cells))
       return false;
-    const FusedArgs A = PerCellArgs(st, nullptr, st.n_cells);
+    FusedArgs A = PerCellArgs(st, nullptr, st.n_cells);
+    A.cell_time = cell_time;
     SolveFusedGroup(s, st, A, dt);
     ReadPerCellResults(st, A, dt, stats, per_cell_status, per_cell_accepted);
     return true;

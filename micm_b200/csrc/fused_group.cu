@@ -99,6 +99,8 @@ namespace micmb
           A.cell_status[cell_of[g]] = c.state;
         if (A.cell_accepted)
           A.cell_accepted[cell_of[g]] = A.ckpt_y ? n_ckpt[g] : c.accepted;
+        if (A.cell_time)
+          A.cell_time[cell_of[g]] = c.t;
         atomicAdd(block_stats + 0, (unsigned long long)c.function_calls);
         atomicAdd(block_stats + 1, (unsigned long long)c.jacobian_updates);
         atomicAdd(block_stats + 2, (unsigned long long)c.number_of_steps);
@@ -248,22 +250,30 @@ namespace micmb
     }
   }  // namespace
 
-  // Cells per block: as many as leave a block for every SM, up to the 8 that share
-  // table words and barriers best, or 32 (a lane per cell) where a cell is so
-  // small that there is nothing to split; halved until a block's cells fit in
-  // shared memory.  Warps per block: by how many items a level of the
-  // mechanism's factorisation has to share out.  Measured, ms: 210 species,
-  // 4,096 cells: G = 2 67.8, 4 66.1, 8 64.9 (8 warps; 16 warps do not fit the
-  // registers); 60 species, 30,000 cells: G = 4 55.7, 8 53.1 (4 warps; 2 warps 61),
-  // 16 55.1, 32 81.8; Chapman, 100,000 cells: G = 8 3.9, 16 2.6, 32 2.0 (1 warp).
+  // Cells per block: as many as leave two blocks for every SM (four from eight cells
+  // on: a block's last cells wait for one another), as long as one block's cells fit
+  // in shared memory.  Warps per block: registers allow eight per SM, shared by the
+  // blocks that share the SM; one where a cell is so small that there is nothing to
+  // split.  Measured, ms: 210 species, 4,096 cells: (cells, warps) = (2, 2) 43.8, (4,
+  // 4) 41.4, (8, 8) 41.3; 60 species, 1,013 cells: (4, 4) 8.1, (4, 2) 9.8, (8, 4) 10.1;
+  // 3,000: (4, 4) 11.6, (8, 4) 10.5, (16, 4) 12.7; 30,000: (8, 4) 53.1, (16, 4) 42.5,
+  // (32, 4) 50.3, (32, 8) 41.6; Chapman, 3,000: (1, 1) 1.08, (4, 1) 0.44, (16, 1) 0.50;
+  // 100,000: (16, 1) 3.6, (32, 1) 2.0, (32, 2) 2.8.
   GroupChoice ChooseGroup(const micmb_solver& s, int64_t n_cells)
   {
     const CompiledMechanism& m = *s.mech;
-    const int32_t most = m.nnz < 128 ? 32 : 8;
-    GroupChoice c{ 1, m.nnz < 128 ? 1 : (m.nnz < 1024 ? 4 : 8) };
-    while (c.G < most && n_cells >= 2 * (int64_t)c.G * s.sm_count &&
-           GroupSharedBytes(s, GroupChoice{ 2 * c.G, c.W }) + 192 * (size_t)c.G + 1024 <= s.smem_optin)
+    const size_t per_cell = GroupSharedBytes(s, GroupChoice{ 1, 1 }) + 96;  // static shared memory included
+    GroupChoice c{ 1, 1 };
+    while (c.G < 32 && n_cells >= (c.G < 8 ? 2 : 4) * (int64_t)c.G * s.sm_count &&
+           2 * c.G * per_cell + 1024 <= s.smem_optin)
       c.G *= 2;
+    if (m.nnz < 128)
+      return c;
+    const int64_t fit = std::max<int64_t>(1, (int64_t)((s.smem_optin + 1024) / (c.G * per_cell + 2048)));
+    const int64_t wanted = (n_cells + (int64_t)c.G * s.sm_count - 1) / ((int64_t)c.G * s.sm_count);
+    const int64_t blocks = std::min(fit, std::max<int64_t>(1, wanted));
+    while (c.W * blocks < 8)
+      c.W *= 2;
     return c;
   }
 

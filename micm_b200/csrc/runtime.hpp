@@ -86,6 +86,7 @@ namespace micmb
     double* ckpt_k;              // [n_cells][max_ckpt][stages][S] stage vectors of each accepted step,
                                  // or null (one-cell-per-thread variant only)
     int32_t max_ckpt;
+    double* cell_time;  // [n_cells] time each cell reached (cell-group kernel), or null
   };
 
   // cells per block and warps of the cell-group kernels
@@ -255,7 +256,7 @@ namespace micmb
   bool LaunchGroupStage(micmb_solver& s, micmb_state& st, GroupStage stage);
   // the plain method on them: per cell, or one step size for all cells; false: not taken
   bool SolvePlainPerCellGroup(micmb_solver& s, micmb_state& st, double dt, micmb_solver_stats* stats,
-                              int32_t* per_cell_status, int32_t* per_cell_accepted);
+                              int32_t* per_cell_status, int32_t* per_cell_accepted, double* cell_time = nullptr);
   bool SolveGlobalGroup(micmb_solver& s, micmb_state& st, double dt, micmb_solver_stats* stats,
                         int32_t* per_cell_status, int32_t* per_cell_accepted);
   int StreamWarpsPerCta(const micmb_solver& s, int slots, int cap, bool lu_shared);
