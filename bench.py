@@ -32,7 +32,7 @@ sys.path.insert(0, ROOT)
 
 METRIC = "cell-solves/s @1M cells, FP64 rtol1e-6 (fused vs plain); adjoint/forward time"
 UNIT = "cell-solves/s"
-KERNEL_OF_VARIANT = {0: "k_fused_stream", 1: "k_fused", 2: "k_fused_thread"}
+KERNEL_OF_VARIANT = {0: "k_group_solve", 1: "k_fused", 2: "k_fused_thread"}
 # workload -> cells per GPU, description, the adjoint timing that goes with it
 # (configuration, cells, checkpoints per cell), host-CPU sample, ncu capture of
 # the fused kernel whose DRAM bytes per cell-solve scale the traffic figure

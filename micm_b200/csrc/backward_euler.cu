@@ -577,8 +577,14 @@ namespace micmb
       }
     }
 
-    // blocks of a cell-group kernel for n cells and the vectors of each; 0 blocks:
-    // the mechanism does not fit
+    // whether n cells are solved by a cell-group kernel: up to where the
+    // thread-per-cell kernels are faster
+    bool GroupFits(const micmb_solver& s, const void* kernel, const GroupChoice& choice, int64_t n)
+    {
+      return n > 0 && GroupFaster(s, n) && GroupBlocksPerSm(s, kernel, choice) > 0;
+    }
+
+    // blocks of a cell-group kernel for n cells and the doubles of each
     struct GroupGrid
     {
       int64_t blocks = 0, slot = 0;
@@ -591,8 +597,7 @@ namespace micmb
       const int per_sm = GroupBlocksPerSm(s, kernel, choice);
       gg.blocks = std::min<int64_t>((int64_t)per_sm * s.sm_count, (n + choice.G - 1) / choice.G);
       gg.slot = doubles_per_cell * choice.G;
-      if (gg.blocks > 0 && st.group_ws.bytes < sizeof(double) * (size_t)(gg.blocks * gg.slot))
-        st.group_ws = DeviceMemory(sizeof(double) * (size_t)(gg.blocks * gg.slot));
+      EnsureGroupWorkspace(st, gg.blocks * gg.slot);
       return gg;
     }
 
@@ -719,9 +724,9 @@ namespace micmb
     {
       const auto& m = *s.mech;
       const int64_t n = st.n_cells;
-      const bool group = n > 0 && GroupVariantApplies(s, n);
-      const GroupChoice choice = group ? ChooseGroup(s, n) : GroupChoice{ 1, 1 };
+      const GroupChoice choice = ChooseGroup(s, n);
       const GroupIterateKernel iterate = GroupIterateFor(choice.G);
+      const bool group = GroupFits(s, reinterpret_cast<const void*>(iterate), choice, n);
       const DevGroup tables = group ? GroupTablesFor(s, choice).dev : DevGroup{};
       GroupGrid gg;
       if (group)
@@ -827,7 +832,9 @@ namespace micmb
     {
       const auto& m = *s.mech;
       const int64_t n = st.n_cells;
-      const bool group = n > 0 && GroupVariantApplies(s, n);
+      const GroupChoice choice = ChooseGroup(s, n);
+      const GroupEulerKernel group_kernel = GroupEulerFor(choice.G);
+      const bool group = GroupFits(s, reinterpret_cast<const void*>(group_kernel), choice, n);
       if (!st.status.p)
         st.status = DeviceMemory(sizeof(int32_t) * std::max<int64_t>(n, 1));
       if (!st.accepted.p)
@@ -849,11 +856,9 @@ namespace micmb
       MICMB_CUDA(cudaMemsetAsync(cbase, 0, 128, stream));
       if (group)
       {
-        const GroupChoice choice = ChooseGroup(s, n);
-        const GroupEulerKernel kernel = GroupEulerFor(choice.G);
-        const GroupGrid gg = PrepareGroup(s, st, reinterpret_cast<const void*>(kernel), choice, n,
+        const GroupGrid gg = PrepareGroup(s, st, reinterpret_cast<const void*>(group_kernel), choice, n,
                                           GroupVectorDoubles(m.S, 0) + m.R);
-        kernel<<<(unsigned)gg.blocks, 32 * choice.W, GroupSharedBytes(s, choice), stream>>>(
+        group_kernel<<<(unsigned)gg.blocks, 32 * choice.W, GroupSharedBytes(s, choice), stream>>>(
             GroupTablesFor(s, choice).dev, P, dt, A, st.group_ws.as<double>(), gg.slot);
         MICMB_CUDA(cudaGetLastError());
       }

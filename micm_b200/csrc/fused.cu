@@ -443,6 +443,7 @@ namespace micmb
     A.cell_time = cell_time;
     SolveFusedGroup(s, st, A, dt);
     ReadPerCellResults(st, A, dt, stats, per_cell_status, per_cell_accepted);
+    MICMB_CUDA(cudaStreamSynchronize(st.stream));  // the plain method returns after the solve
     return true;
   }
 }  // namespace micmb

@@ -364,9 +364,24 @@ namespace micmb
     return per_sm;
   }
 
+  void EnsureGroupWorkspace(micmb_state& st, int64_t doubles)
+  {
+    if (st.group_ws.bytes >= sizeof(double) * (size_t)doubles)
+      return;
+    // a captured solve holds the old workspace's address
+    if (st.graph_exec)
+    {
+      MICMB_CUDA(cudaGraphExecDestroy(st.graph_exec));
+      st.graph_exec = nullptr;
+    }
+    st.group_ws = DeviceMemory(sizeof(double) * (size_t)doubles);
+  }
+
   bool GroupVariantApplies(const micmb_solver& s, int64_t n_cells)
   {
-    if (!GroupApplies(*s.mech))
+    // the register-blocked schedules, asked for by the environment, are the
+    // thread-per-cell kernels'
+    if (!GroupApplies(*s.mech) || s.dev.has_blocked)
       return false;
     const GroupChoice choice = ChooseGroup(s, n_cells);
     return GroupBlocksPerSm(s, reinterpret_cast<const void*>(SolveKernelFor(choice.G)), choice) > 0;
@@ -411,8 +426,7 @@ namespace micmb
     const int64_t grid =
         std::max<int64_t>(1, std::min<int64_t>((int64_t)per_sm * s.sm_count, (A.n_cells + choice.G - 1) / choice.G));
     const int64_t slot = (GroupVectorDoubles(s.mech->S, s.params.stages) + s.mech->R) * choice.G;
-    if (st.group_ws.bytes < sizeof(double) * (size_t)(grid * slot))
-      st.group_ws = DeviceMemory(sizeof(double) * (size_t)(grid * slot));
+    EnsureGroupWorkspace(st, grid * slot);
     kernel<<<(unsigned)grid, 32 * choice.W, GroupSharedBytes(s, choice), st.stream>>>(
         t.dev, s.params, step_bounds(s.params, dt), A, st.group_ws.as<double>(), slot);
     MICMB_CUDA(cudaGetLastError());

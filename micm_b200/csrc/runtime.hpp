@@ -242,6 +242,8 @@ namespace micmb
   int GroupBlocksPerSm(const micmb_solver& s, const void* kernel, const GroupChoice& choice);
   bool GroupVariantApplies(const micmb_solver& s, int64_t n_cells);
   int32_t GroupCellsPerSm(const micmb_solver& s);
+  // st.group_ws of at least that many doubles
+  void EnsureGroupWorkspace(micmb_state& st, int64_t doubles);
   bool GroupFaster(const micmb_solver& s, int64_t n_cells);  // than the one-cell-per-thread kernel
   bool GroupFasterThanStages(const micmb_solver& s, int64_t n_cells);  // than the plain per-stage kernels
   void SolveFusedGroup(micmb_solver& s, micmb_state& st, const FusedArgs& A, double dt);
