@@ -3,8 +3,8 @@
 //
 // The forward solve (SolveFused with checkpointing) stores, for every accepted
 // step n of every cell, the starting state y_n, the step size H_n and (where
-// memory allows) the stage vectors K_s.  The backward sweep, one cell per
-// thread, then walks each cell's steps backwards.  For step n it rebuilds
+// memory allows) the stage vectors K_s.  The backward sweep, on cell groups in
+// shared memory or one cell per thread, then walks each cell's steps backwards.  For step n it rebuilds
 // alpha I - J(y_n) and its LU factor, takes the stored stages or recomputes
 // them exactly as the forward pass did (same routines, so the same bits), and
 // applies the transposed step with the step size held fixed:
@@ -22,6 +22,7 @@
 // so d w_r / d log k_r = w_r).  The same recurrences, in the same order, are
 // restated on the CPU by the test oracle (om_adjoint_per_cell).
 #include "runtime.hpp"
+#include "group.cuh"
 
 #include <algorithm>
 #include <vector>
@@ -52,7 +53,7 @@ namespace micmb
       double* ybar0;                 // vector layout [S]
       double* kbar;                  // [cell][R]
       int32_t* next_cell;
-      const int32_t* order;          // cells in decreasing step count (thread kernel), or null
+      const int32_t* order;          // cells in decreasing step count, or null
     };
 
     // ---- one cell per thread, private working sets in global memory ----
@@ -465,6 +466,364 @@ namespace micmb
       }
     }
 
+    // ---- cell groups: a block sweeps G cells in lockstep, their factors in shared memory ----
+
+    // nu_r . v for elements v0 + column
+    template<int G>
+    __device__ __forceinline__ double nu_dot_g(const DevMech& M, int32_t r, const GroupThread<G>& X, int32_t v0)
+    {
+      double s = 0.0;
+      for (int32_t i = M.prod_start[r]; i < M.prod_start[r + 1]; ++i)
+        s += M.prod_yield[i] * X[v0 + M.prod_ids[i]];
+      for (int32_t i = M.react_start[r]; i < M.react_start[r + 1]; ++i)
+        s -= X[v0 + M.react_ids[i]];
+      return s;
+    }
+
+    // a reaction's reactants (rate_desc), their values in V and the products of the others
+    struct Reactants
+    {
+      int32_t id[3], n;
+      double y[3], others[3];
+    };
+    template<int G>
+    __device__ __forceinline__ Reactants reactants_of(const DevMech& M, const DevGroup& P, const GroupThread<G>& X,
+                                                      int32_t r)
+    {
+      Reactants a;
+      const int4 d = M.rate_desc[r];
+      a.id[0] = d.x;
+      a.id[1] = d.y;
+      a.id[2] = d.z;
+      a.n = 0;
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+      {
+        a.y[q] = a.id[q] < M.S ? X[P.v0 + a.id[q]] : 1.0;
+        a.n += a.id[q] < M.S ? 1 : 0;
+      }
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+      {
+        double v = 1.0;
+#pragma unroll
+        for (int o = 0; o < 3; ++o)
+          if (o != q && o < a.n)
+            v *= a.y[o];
+        a.others[q] = v;
+      }
+      return a;
+    }
+
+    // kb[r] += (nu_r . g) w_r, and the reaction's terms of J^T g to element first + q
+    // for reactant q (state in V, g in G2).  What the thread kernel skips is -0,
+    // which leaves every sum as it is.
+    template<int G>
+    __device__ __forceinline__ void project(const Reactants& a, double k, double c, const GroupThread<G>& X,
+                                            const int32_t (&to)[3], double& kb)
+    {
+      if (c != 0.0)
+        kb += c * (k * (((1.0 * a.y[0]) * a.y[1]) * a.y[2]));
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        if (q < a.n)
+          X[to[q]] = c != 0.0 ? c * k * a.others[q] : -0.0;
+    }
+
+    template<int G>
+    __device__ __forceinline__ void group_vjp(const DevMech& M, const DevGroup& P, const GroupThread<G>& X,
+                                              const double* kk, double* kb)
+    {
+      for (int32_t r = X.lane; r < P.R; r += X.lanes)
+      {
+        const int32_t first = P.slot + M.react_start[r];
+        const int32_t to[3] = { first, first + 1, first + 2 };
+        project<G>(reactants_of(M, P, X, r), kk[(int64_t)r * G], nu_dot_g(M, r, X, P.g2), X, to, kb[(int64_t)r * G]);
+      }
+    }
+
+    // Contributions of a whole step at its start: stage < 0, J^T Gbar_0; else the
+    // second-order terms of that stage (Rbar in G2, K in the inv elements, which no
+    // solve needs any more).
+    template<int G>
+    __device__ __forceinline__ void group_step_terms(const DevMech& M, const DevGroup& P, const GroupThread<G>& X,
+                                                     int32_t stage, const double* kk, double* kb)
+    {
+      for (int32_t r = X.lane; r < P.R; r += X.lanes)
+      {
+        const double k = kk[(int64_t)r * G], c = nu_dot_g(M, r, X, P.g2);
+        const Reactants a = reactants_of(M, P, X, r);
+        int32_t i = P.step_start[r];
+        auto element = [&](int32_t e) { return e < P.nnz ? e : P.slot + e - P.nnz; };
+        if (stage < 0)
+        {
+          const int32_t to[3] = { element(i), element(i + 1), element(i + 2) };
+          project<G>(a, k, c, X, to, kb[(int64_t)r * G]);
+          continue;
+        }
+        i += a.n + stage * a.n * (a.n - 1);
+        double kv[3], gk = 0.0;
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+        {
+          kv[q] = q < a.n ? X[P.inv + a.id[q]] : 0.0;
+          if (q < a.n)
+            gk += k * a.others[q] * kv[q];
+        }
+        if (c != 0.0)
+          kb[(int64_t)r * G] += c * gk;
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+#pragma unroll
+          for (int o = 0; o < 3; ++o)
+            if (q != o && q < a.n && o < a.n)
+            {
+              const double v = a.n == 3 ? 1.0 * a.y[3 - q - o] : 1.0;
+              X[element(i++)] = c != 0.0 ? c * k * v * kv[q] : -0.0;
+            }
+      }
+    }
+
+    // The backward sweep with stored stages: the thread kernel's sums, in the same
+    // order, so the same bits.  Per step one factorisation and a transposed solve per
+    // stage as in the forward kernel, and per evaluation a pass over the reactions
+    // whose contributions go to shared memory and are gathered per species, as the
+    // sums of a species have to keep the reactions' order.  Bound by the solves'
+    // dependency levels, as the forward kernel; the stages' vectors (Kbar, Gbar,
+    // Rbar) stay in L2.  The thread kernel, with a working set per thread in HBM, is
+    // bound by latency below some 100,000 cells.  Measured, forward and sweep of
+    // 8,192 cells of 60 species: 347 -> 54 ms; 16,384 of 210: 1,608 -> 500; 2,048 of
+    // 600: 5,706 -> 611.
+    template<int G>
+    __global__ void __launch_bounds__(256, 1)
+        k_adjoint_group(DevMech M, DevGroup P, DevParams D, AdjArgs A, double* ws, int64_t slot_doubles)
+    {
+      extern __shared__ __align__(16) double shared[];
+      __shared__ int64_t cell_of[G];
+      __shared__ int32_t step[G];  // checkpoint being swept; -1: none
+      const GroupThread<G> X(shared);
+      const int32_t g = threadIdx.x & (G - 1), S = P.S, L = A.L, ns = D.stages;
+      double* w = ws + (int64_t)blockIdx.x * slot_doubles + g;
+      auto take = [&](int64_t n) {
+        double* at = w;
+        w += n * G;
+        return at;
+      };
+      double *yv = take(S), *yb = take(S), *Kb = take((int64_t)ns * S), *Gb = take((int64_t)ns * S),
+             *Rb = take((int64_t)ns * S), *kk = take(P.R), *kb = take(P.R);
+      auto at = [&](double* v, int32_t st, int32_t i) -> double& { return v[((int64_t)st * S + i) * G]; };
+      if (X.lane == 0)
+      {
+        X[P.zero] = 0.0;
+        X[P.one] = 1.0;
+        X[P.trash] = 1.0;
+      }
+      for (int32_t i = X.lane; i < S; i += X.lanes)
+      {
+        yv[(int64_t)i * G] = yb[(int64_t)i * G] = 0.0;
+        for (int32_t st = 0; st < ns; ++st)
+          at(Kb, st, i) = at(Gb, st, i) = at(Rb, st, i) = 0.0;
+      }
+      for (int32_t r = X.lane; r < P.R; r += X.lanes)
+        kk[(int64_t)r * G] = kb[(int64_t)r * G] = 0.0;
+      constexpr int32_t kWants = -2, kNone = -1;
+      if (threadIdx.x < G)
+        step[g] = kWants;
+      auto finish = [&]() {
+        double* out = A.ybar0 + cell_base(cell_of[g], L, S);
+        for (int32_t i = X.lane; i < S; i += X.lanes)
+          out[(int64_t)i * L] = yb[(int64_t)i * G];
+        for (int32_t r = X.lane; r < P.R; r += X.lanes)
+          A.kbar[(size_t)cell_of[g] * P.R + r] = kb[(int64_t)r * G];
+      };
+      for (;;)
+      {
+        // new cells; those without a step are done at once
+        __syncthreads();
+        while (__syncthreads_or(step[g] == kWants))
+        {
+          const bool wants = step[g] == kWants;
+          __syncthreads();
+          if (threadIdx.x < G && wants)
+          {
+            const int64_t k = atomicAdd(A.next_cell, 1);
+            cell_of[g] = k < A.n_cells ? (A.order ? A.order[k] : k) : -1;
+          }
+          __syncthreads();
+          const int64_t c = cell_of[g];
+          const int32_t n_ck = wants && c >= 0 ? A.n_ckpt[c] : 0;
+          if (wants && c >= 0)
+          {
+            const double* k = A.rate_constants + cell_base(c, L, P.R);
+            for (int32_t r = X.lane; r < P.R; r += X.lanes)
+            {
+              kk[(int64_t)r * G] = k[(int64_t)r * L];
+              kb[(int64_t)r * G] = 0.0;
+            }
+            if (n_ck == 0)
+            {
+              const size_t by = cell_base(c, L, S);
+              for (int32_t i = X.lane; i < S; i += X.lanes)
+                yb[(int64_t)i * G] = (A.y0[by + (size_t)i * L] < 0.0) ? 0.0 : A.ybar_final[by + (size_t)i * L];
+              finish();
+            }
+          }
+          __syncthreads();
+          if (threadIdx.x < G && wants)
+            step[g] = c < 0 ? kNone : (n_ck > 0 ? n_ck - 1 : kWants);
+          __syncthreads();
+        }
+        const int32_t n = step[g];
+        const bool live = n >= 0;
+        if (!__syncthreads_or(live))
+          break;
+        const int64_t c = live ? cell_of[g] : 0;
+        const size_t row = (size_t)c * A.max_ckpt + (live ? n : 0);
+        const double* yc = A.ckpt_y + row * S;
+        const double* kc = A.ckpt_k + row * (size_t)ns * S;
+        const double H = live ? A.ckpt_h[row] : 1.0;
+        // the step's factor
+        for (int32_t i = X.lane; i < S; i += X.lanes)
+          X[P.v0 + i] = yv[(int64_t)i * G] = live ? yc[i] : 0.0;
+        __syncthreads();
+        group_drates<G>(P, X, kk, G);
+        __syncthreads();
+        run_gather<G>(P.jacobian, X, 1.0 / (H * D.gamma0));
+        __syncthreads();
+        if (X.lane == 0)
+          X[P.inv + S] = 1.0;  // the Jacobian rates were there
+        run_levels<G, true>(P.lu, X, P);
+        __syncthreads();
+        if (X.lane == 0)
+          X[P.trash] = 1.0;  // idle lanes left what is slow to divide
+        const bool last_step = live && n == A.n_ckpt[c] - 1;
+        for (int32_t i = X.lane; i < S; i += X.lanes)
+        {
+          if (last_step)
+          {
+            double v = yv[(int64_t)i * G];
+            for (int32_t st = 0; st < ns; ++st)
+              v += D.m[st] * kc[(int64_t)st * S + i];
+            yb[(int64_t)i * G] = (v < 0.0) ? 0.0 : A.ybar_final[cell_base(c, L, S) + (size_t)i * L];
+          }
+          const double b = live ? yb[(int64_t)i * G] : 0.0;
+          for (int32_t st = 0; st < ns; ++st)
+          {
+            at(Kb, st, i) = D.m[st] * b;
+            at(Gb, st, i) = 0.0;
+          }
+        }
+        for (int32_t st = ns - 1; st >= 0; --st)
+        {
+          const int32_t sc = st * (st - 1) / 2;
+          for (int32_t i = X.lane; i < S; i += X.lanes)
+            X[P.v0 + i] = at(Kb, st, i);
+          __syncthreads();
+          run_levels<G, false>(P.solve, X, P);
+          __syncthreads();
+          double coh[kMaxAdjStages];
+          for (int32_t j = 0; j < st; ++j)
+            coh[j] = D.c[sc + j] / H;
+          const bool fresh = st > 0 && D.new_f[st];
+          for (int32_t i = X.lane; i < S; i += X.lanes)
+          {
+            const double v = X[P.v0 + i];
+            at(Rb, st, i) = v;
+            const double gb = at(Gb, st, i) + v;
+            at(Gb, st, i) = gb;
+            for (int32_t j = 0; j < st; ++j)
+              at(Kb, j, i) += coh[j] * v;
+            if (fresh)
+            {
+              double y = yv[(int64_t)i * G];
+              for (int32_t j = 0; j < st; ++j)
+                y += D.a[sc + j] * (live ? kc[(int64_t)j * S + i] : 0.0);
+              X[P.v0 + i] = y;
+              X[P.g2 + i] = gb;
+            }
+            else if (st > 0)
+              at(Gb, st - 1, i) += gb;
+          }
+          if (!fresh)
+            continue;
+          __syncthreads();
+          group_vjp<G>(M, P, X, kk, kb);
+          __syncthreads();
+          run_gather<G>(P.forcing, X, 0.0);
+          __syncthreads();
+          for (int32_t i = X.lane; i < S; i += X.lanes)
+          {
+            const double t = X[P.v0 + i];
+            yb[(int64_t)i * G] += t;
+            for (int32_t j = 0; j < st; ++j)
+              at(Kb, j, i) += D.a[sc + j] * t;
+          }
+        }
+        // the terms at the step's start
+        for (int32_t i = X.lane; i < S; i += X.lanes)
+        {
+          X[P.v0 + i] = yv[(int64_t)i * G];
+          X[P.g2 + i] = at(Gb, 0, i);
+        }
+        __syncthreads();
+        group_step_terms<G>(M, P, X, -1, kk, kb);
+        for (int32_t st = 0; st < ns; ++st)
+        {
+          __syncthreads();
+          for (int32_t i = X.lane; i < S; i += X.lanes)
+          {
+            X[P.g2 + i] = at(Rb, st, i);
+            X[P.inv + i] = live ? kc[(int64_t)st * S + i] : 0.0;
+          }
+          __syncthreads();
+          group_step_terms<G>(M, P, X, st, kk, kb);
+        }
+        __syncthreads();  // the state in V has been read
+        for (int32_t i = X.lane; i < S; i += X.lanes)
+          X[P.v0 + i] = yb[(int64_t)i * G];
+        __syncthreads();
+        run_gather<G, true>(P.step, X, 0.0);
+        __syncthreads();
+        for (int32_t i = X.lane; i < S; i += X.lanes)
+          yb[(int64_t)i * G] = X[P.v0 + i];
+        __syncthreads();
+        if (live && n == 0)
+          finish();
+        if (threadIdx.x < G && live)
+          step[g] = n > 0 ? n - 1 : kWants;
+      }
+    }
+
+    using AdjGroupKernel = void (*)(DevMech, DevGroup, DevParams, AdjArgs, double*, int64_t);
+
+    // Where the cell-group sweep is the faster one.  Measured, with the forward solve,
+    // ms, cell groups / one cell per thread: Chapman 16,384 cells 3.9 / 4.0, 50,000
+    // 9.4 / 9.1; 60 species 65,536 345 / 596, 131,072 691 / 799, 262,144 1,381 / 1,316;
+    // 210 species (8 cells per SM) 49,152 1,504 / 2,177, and from the slopes equal at
+    // about 97,000.  For small
+    // mechanisms, whose blocks are single warps, the line lies lower.
+    bool SweepGroupFaster(const micmb_solver& s, int64_t n)
+    {
+      if (!GroupFaster(s, n))
+        return false;
+      if (s.mech->nnz < 128)
+        return n <= (int64_t)s.sm_count * 128;
+      return n <= std::min<int64_t>((int64_t)s.sm_count * 1024, 12288 * (int64_t)GroupCellsPerSm(s));
+    }
+
+    AdjGroupKernel AdjointGroupFor(int32_t G)
+    {
+      switch (G)
+      {
+        case 1: return k_adjoint_group<1>;
+        case 2: return k_adjoint_group<2>;
+        case 4: return k_adjoint_group<4>;
+        case 8: return k_adjoint_group<8>;
+        case 16: return k_adjoint_group<16>;
+        default: return k_adjoint_group<32>;
+      }
+    }
+
     // 96 registers, 5 blocks of 128 per SM, no spills.  A full-occupancy build
     // (32 registers, as the forward kernel's fastest) measured slower here:
     // 1.38 s against 1.16 s on 131,072 cells of the 60-species mechanism, and
@@ -561,7 +920,7 @@ namespace micmb
     }
   }  // namespace
 
-  // one cell per thread: per-thread working sets in global memory, no atomics
+  // cell groups, or one cell per thread with working sets in global memory; no atomics
   void LaunchAdjointThread(micmb_solver& s, micmb_state& st, int32_t max_ckpt, int64_t begin, int64_t count)
   {
     const auto& m = *s.mech;
@@ -576,9 +935,6 @@ namespace micmb
     const int64_t n = count;
     int64_t grid = (int64_t)per_sm * s.sm_count;
     grid = std::max<int64_t>(1, std::min<int64_t>(grid, (n + 127) / 128));
-    const int64_t doubles = grid * 128 * (int64_t)T.per_slot;
-    if (!st.thread_ws.p || st.thread_ws.bytes < (size_t)doubles * sizeof(double))
-      st.thread_ws = DeviceMemory((size_t)doubles * sizeof(double));
     AdjArgs A = ChunkArgs(s, st, max_ckpt, begin, count);
     MICMB_CUDA(cudaMemsetAsync(A.next_cell, 0, 8, st.stream));
     if (n > 0)
@@ -596,6 +952,24 @@ namespace micmb
       k_step_scatter<<<blocks, 256, 0, st.stream>>>(A.n_ckpt, n, max_ckpt, bins, order);
       MICMB_CUDA(cudaGetLastError());
       A.order = order;
+      const GroupChoice choice = ChooseGroup(s, n, s.params.stages);
+      const AdjGroupKernel group = AdjointGroupFor(choice.G);
+      const int group_blocks = A.ckpt_k && SweepGroupFaster(s, n)
+                                   ? GroupBlocksPerSm(s, reinterpret_cast<const void*>(group), choice)
+                                   : 0;
+      if (group_blocks > 0)
+      {
+        const int64_t blocks = std::min<int64_t>((int64_t)group_blocks * s.sm_count, (n + choice.G - 1) / choice.G);
+        const int64_t slot = ((int64_t)m.S * (2 + 3 * s.params.stages) + 2 * (int64_t)m.R) * choice.G;
+        EnsureGroupWorkspace(st, blocks * slot);
+        group<<<(unsigned)blocks, 32 * choice.W, GroupSharedBytes(s, choice), st.stream>>>(
+            s.dev, GroupTablesFor(s, choice).dev, s.params, A, st.group_ws.as<double>(), slot);
+        MICMB_CUDA(cudaGetLastError());
+        return;
+      }
+      const int64_t doubles = grid * 128 * (int64_t)T.per_slot;
+      if (!st.thread_ws.p || st.thread_ws.bytes < (size_t)doubles * sizeof(double))
+        st.thread_ws = DeviceMemory((size_t)doubles * sizeof(double));
       kernel<<<(unsigned)grid, 128, 0, st.stream>>>(s.dev, s.params, A, T, st.thread_ws.as<double>());
       MICMB_CUDA(cudaGetLastError());
     }

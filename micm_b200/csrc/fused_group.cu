@@ -259,11 +259,11 @@ namespace micmb
   // 3,000: (4, 4) 11.6, (8, 4) 10.5, (16, 4) 12.7; 30,000: (8, 4) 53.1, (16, 4) 42.5,
   // (32, 4) 50.3, (32, 8) 41.6; Chapman, 3,000: (1, 1) 1.08, (4, 1) 0.44, (16, 1) 0.50;
   // 100,000: (16, 1) 3.6, (32, 1) 2.0, (32, 2) 2.8.
-  GroupChoice ChooseGroup(const micmb_solver& s, int64_t n_cells)
+  GroupChoice ChooseGroup(const micmb_solver& s, int64_t n_cells, int32_t sweep_stages)
   {
     const CompiledMechanism& m = *s.mech;
-    const size_t per_cell = GroupSharedBytes(s, GroupChoice{ 1, 1 }) + 96;  // static shared memory included
-    GroupChoice c{ 1, 1 };
+    const size_t per_cell = GroupSharedBytes(s, GroupChoice{ 1, 1, sweep_stages }) + 96;  // static shared memory included
+    GroupChoice c{ 1, 1, sweep_stages };
     while (c.G < 32 && n_cells >= (c.G < 8 ? 2 : 4) * (int64_t)c.G * s.sm_count &&
            2 * c.G * per_cell + 1024 <= s.smem_optin)
       c.G *= 2;
@@ -281,9 +281,9 @@ namespace micmb
   {
     std::lock_guard<std::mutex> lock(s.group_mutex);
     for (const auto& t : s.group)
-      if (t->choice.G == choice.G && t->choice.W == choice.W)
+      if (t->choice.G == choice.G && t->choice.W == choice.W && t->choice.sweep_stages == choice.sweep_stages)
         return *t;
-    const GroupProgram p = BuildGroupProgram(*s.mech, choice.G, choice.W);
+    const GroupProgram p = BuildGroupProgram(*s.mech, choice.G, choice.W, choice.sweep_stages);
     auto t = std::make_unique<GroupTables>();
     t->choice = choice;
     std::vector<char> bytes;
@@ -308,6 +308,8 @@ namespace micmb
       return o;
     };
     const Offsets of = add_phase(p.forcing), oj = add_phase(p.jacobian), ol = add_phase(p.lu), os = add_phase(p.solve);
+    const Offsets ostep = add_phase(p.step);
+    const size_t ostart = add(p.step_start);
     const size_t orate = add(p.rate), odrate = add(p.drate);
     t->memory = DeviceMemory(bytes.size());
     MICMB_CUDA(cudaMemcpy(t->memory.p, bytes.data(), bytes.size(), cudaMemcpyHostToDevice));
@@ -336,11 +338,15 @@ namespace micmb
     g.w0 = p.layout.w0;
     g.inv = p.layout.inv;
     g.rate = p.layout.rate;
+    g.g2 = p.layout.g2;
+    g.slot = p.layout.slot;
     g.elements = p.layout.elements;
     g.forcing = phase(of);
     g.jacobian = phase(oj);
     g.lu = phase(ol);
     g.solve = phase(os);
+    g.step = phase(ostep);
+    g.step_start = reinterpret_cast<const int32_t*>(b + ostart);
     g.rate_tab = reinterpret_cast<const uint2*>(b + orate);
     g.drate_tab = reinterpret_cast<const uint2*>(b + odrate);
     s.group.push_back(std::move(t));
@@ -349,7 +355,7 @@ namespace micmb
 
   size_t GroupSharedBytes(const micmb_solver& s, const GroupChoice& choice)
   {
-    return sizeof(double) * (size_t)MakeGroupLayout(*s.mech).elements * choice.G;
+    return sizeof(double) * (size_t)MakeGroupLayout(*s.mech, choice.sweep_stages).elements * choice.G;
   }
 
   int GroupBlocksPerSm(const micmb_solver& s, const void* kernel, const GroupChoice& choice)

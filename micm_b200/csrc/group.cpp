@@ -333,7 +333,18 @@ namespace micmb
     }
   }  // namespace
 
-  GroupLayout MakeGroupLayout(const CompiledMechanism& m)
+  namespace
+  {
+    // contributions of reaction r in a step: first derivatives per reactant, then
+    // per stage the pairs of different reactants
+    int32_t Contributions(const CompiledMechanism& m, int32_t r, int32_t stages)
+    {
+      const int32_t n = m.react_start[r + 1] - m.react_start[r];
+      return n + stages * n * (n - 1);
+    }
+  }  // namespace
+
+  GroupLayout MakeGroupLayout(const CompiledMechanism& m, int32_t sweep_stages)
   {
     GroupLayout L;
     const int32_t n_info = (int32_t)m.info_rxn.size();
@@ -344,7 +355,17 @@ namespace micmb
     L.w0 = L.trash + 1;
     L.inv = L.w0;
     L.rate = L.inv + m.S + 1;
-    L.elements = L.w0 + std::max(n_info, m.S + 1 + std::max(m.R, m.S));
+    L.g2 = L.rate;
+    L.slot = L.g2 + m.S;
+    int32_t vectors = m.S + 1 + std::max(m.R, m.S);
+    if (sweep_stages > 0)
+    {
+      int32_t total = 0;
+      for (int32_t r = 0; r < m.R; ++r)
+        total += Contributions(m, r, sweep_stages);
+      vectors = 2 * m.S + 1 + std::max((int32_t)m.react_ids.size(), total - m.nnz);
+    }
+    L.elements = L.w0 + std::max(n_info, vectors);
     return L;
   }
 
@@ -354,14 +375,14 @@ namespace micmb
            !m.rate_desc.empty();
   }
 
-  GroupProgram BuildGroupProgram(const CompiledMechanism& m, int32_t G, int32_t W)
+  GroupProgram BuildGroupProgram(const CompiledMechanism& m, int32_t G, int32_t W, int32_t sweep_stages)
   {
     if (!GroupApplies(m))
       throw std::runtime_error("group program: the mechanism has none");
     GroupProgram P;
     P.G = G;
     P.W = W;
-    const GroupLayout L = P.layout = MakeGroupLayout(m);
+    const GroupLayout L = P.layout = MakeGroupLayout(m, sweep_stages);
     const int32_t ipw = 32 / G;
 
     // products: rate_desc / drate_desc pad with column S + 1
@@ -379,7 +400,46 @@ namespace micmb
       P.drate.push_back(vec(d[2]) | (vec(d[3]) << 16));
     }
 
-    P.forcing = GatherPhase(m.f_start, m.f_rxn, m.f_coef, L.rate, L.v0, L, G, W, {});
+    if (sweep_stages == 0)
+      P.forcing = GatherPhase(m.f_start, m.f_rxn, m.f_coef, L.rate, L.v0, L, G, W, {});
+    else
+    {
+      // every species' contributions in the order of the one-cell-per-thread sweep:
+      // by reaction, first derivatives by reactant, then by stage the pairs (q, o)
+      // of different reactants, which go to reactant o
+      std::vector<std::vector<int32_t>> first(m.S), all(m.S);
+      int32_t at = 0;
+      for (int32_t r = 0; r < m.R; ++r)
+      {
+        const int32_t r0 = m.react_start[r], n = m.react_start[r + 1] - r0;
+        P.step_start.push_back(at);
+        auto add = [&](int32_t reactant) {
+          all[m.react_ids[r0 + reactant]].push_back(at < m.nnz ? at : L.slot + at - m.nnz);
+          ++at;
+        };
+        for (int32_t q = 0; q < n; ++q)
+        {
+          first[m.react_ids[r0 + q]].push_back(L.slot + r0 + q);
+          add(q);
+        }
+        for (int32_t st = 0; st < sweep_stages; ++st)
+          for (int32_t q = 0; q < n; ++q)
+            for (int32_t o = 0; o < n; ++o)
+              if (o != q)
+                add(o);
+      }
+      auto phase = [&](const std::vector<std::vector<int32_t>>& of) {
+        std::vector<int32_t> start{ 0 }, element;
+        for (const auto& list : of)
+        {
+          element.insert(element.end(), list.begin(), list.end());
+          start.push_back((int32_t)element.size());
+        }
+        return GatherPhase(start, element, std::vector<double>(element.size(), 1.0), 0, L.v0, L, G, W, {});
+      };
+      P.forcing = phase(first);
+      P.step = phase(all);
+    }
     std::vector<char> diag(m.nnz, 0);
     for (int32_t i = 0; i < m.S; ++i)
       diag[m.diag_pos[i]] = 1;
@@ -401,7 +461,9 @@ namespace micmb
     Emit(P.lu, lu.lists, L, G, false, true);
 
     LevelLists solve(W);
-    for (const LevelSchedule* s : { &m.fwd_serial, &m.bwd_serial })
+    const LevelSchedule* const order[2] = { sweep_stages ? &m.fwd_t_serial : &m.fwd_serial,
+                                            sweep_stages ? &m.bwd_t_serial : &m.bwd_serial };
+    for (const LevelSchedule* s : order)
       solve.Add(*s, false, ipw, L.one, [&](const Piece& p) {
         Sum u;
         u.target = L.v0 + s->item_target[p.item];

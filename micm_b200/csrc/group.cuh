@@ -23,8 +23,9 @@ namespace micmb
   struct DevGroup
   {
     int32_t S, R, n_info, nnz;
-    int32_t zero, one, v0, trash, w0, inv, rate, elements;
-    DevGroupPhase forcing, jacobian, lu, solve;
+    int32_t zero, one, v0, trash, w0, inv, rate, g2, slot, elements;
+    DevGroupPhase forcing, jacobian, lu, solve, step;
+    const int32_t* step_start;
     const uint2* rate_tab;
     const uint2* drate_tab;
   };

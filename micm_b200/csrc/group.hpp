@@ -28,9 +28,15 @@ namespace micmb
     int32_t w0;         // Jacobian rates (n_info), later inv and the rates
     int32_t inv;        // S: 1 / u_ii, and 1.0 as the trash element's
     int32_t rate;       // max(R, S): reaction rates, then the scaled squared errors
+    int32_t g2;         // backward sweep, in place of the rates: S, what reactions project on
+    int32_t slot;       // and their contributions, one per (reaction, reactant) ...
     int32_t elements;
   };
-  GroupLayout MakeGroupLayout(const CompiledMechanism& m);
+  // sweep_stages: 0, or the stages of the adjoint's backward sweep.  The
+  // contributions of a whole step, of which there are more, begin in the factor,
+  // which is no longer needed then: contribution i is element i below nnz, and
+  // slot + i - nnz from there on.
+  GroupLayout MakeGroupLayout(const CompiledMechanism& m, int32_t sweep_stages = 0);
 
   // What becomes of a unit's sums v.  Level phases: kGroupPlain stores v * [aux] in
   // the LU and v in the solves; kGroupPivot stores v and [aux] = 1 / v in the LU, and
@@ -71,8 +77,11 @@ namespace micmb
   {
     int32_t G = 0, W = 0;
     GroupLayout layout{};
-    GroupPhase forcing, jacobian, lu;
-    GroupPhase solve;  // forward, then backward substitution
+    GroupPhase forcing;  // sweep: one evaluation's contributions to each species, into V
+    GroupPhase jacobian, lu;
+    GroupPhase solve;  // forward, then backward substitution (sweep: with the transposed factors)
+    GroupPhase step;   // sweep: a step's contributions to each species, added to V
+    std::vector<int32_t> step_start;  // sweep: [R] a reaction's first contribution
     std::vector<uint32_t> rate;   // [2R]: reactant elements a | b << 16, c (one where there are fewer)
     std::vector<uint32_t> drate;  // [2 n_info]: rate column | a << 16, b | c << 16
   };
@@ -80,5 +89,5 @@ namespace micmb
   // Whether the mechanism has group work lists at all (16-bit elements, at most
   // three reactants, no algebraic constraints).
   bool GroupApplies(const CompiledMechanism& m);
-  GroupProgram BuildGroupProgram(const CompiledMechanism& m, int32_t G, int32_t W);
+  GroupProgram BuildGroupProgram(const CompiledMechanism& m, int32_t G, int32_t W, int32_t sweep_stages = 0);
 }  // namespace micmb

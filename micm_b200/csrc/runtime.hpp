@@ -93,6 +93,7 @@ namespace micmb
   struct GroupChoice
   {
     int32_t G, W;
+    int32_t sweep_stages = 0;  // of the adjoint's backward sweep; 0: the forward kernels
   };
   struct GroupTables
   {
@@ -236,7 +237,7 @@ namespace micmb
   bool SolveFusedThread(micmb_solver& s, micmb_state& st, const FusedArgs& A, double dt);
   // cell-group kernels: the block shape for n_cells cells, its work lists on the
   // device, dynamic shared memory, resident blocks (0: the cells do not fit)
-  GroupChoice ChooseGroup(const micmb_solver& s, int64_t n_cells);
+  GroupChoice ChooseGroup(const micmb_solver& s, int64_t n_cells, int32_t sweep_stages = 0);
   const GroupTables& GroupTablesFor(micmb_solver& s, const GroupChoice& choice);
   size_t GroupSharedBytes(const micmb_solver& s, const GroupChoice& choice);
   int GroupBlocksPerSm(const micmb_solver& s, const void* kernel, const GroupChoice& choice);

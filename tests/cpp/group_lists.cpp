@@ -23,9 +23,9 @@ namespace
     std::vector<double> E;  // the cell's elements
     int64_t bad = 0;
 
-    Checker(const CompiledMechanism& mech, int G, int warps)
+    Checker(const CompiledMechanism& mech, int G, int warps, int sweep_stages)
         : m(mech),
-          p(BuildGroupProgram(mech, G, warps)),
+          p(BuildGroupProgram(mech, G, warps, sweep_stages)),
           L(p.layout),
           ipw(32 / G),
           W(warps),
@@ -186,12 +186,13 @@ namespace
 }  // namespace
 
 // number of faults; -1: the mechanism has no group work lists
-extern "C" int64_t check_group_lists(const micmb_mechanism_desc* desc, int32_t G, int32_t W)
+extern "C" int64_t check_group_lists(const micmb_mechanism_desc* desc, int32_t G, int32_t W,
+                                     int32_t sweep_stages)
 {
   const CompiledMechanism m = Compile(*desc);
   if (!GroupApplies(m))
     return -1;
-  Checker c(m, G, W);
+  Checker c(m, G, W, sweep_stages);
   const GroupLayout& L = c.L;
   std::mt19937_64 rng(5);
   std::uniform_real_distribution<double> uniform(0.5, 1.5);
@@ -232,7 +233,9 @@ extern "C" int64_t check_group_lists(const micmb_mechanism_desc* desc, int32_t G
   same(c.E.data() + L.inv, inv);
 
   c.RunLevels(c.p.solve, false);
-  for (const LevelSchedule* s : { &m.fwd_serial, &m.bwd_serial })
+  const LevelSchedule* const order[2] = { sweep_stages ? &m.fwd_t_serial : &m.fwd_serial,
+                                          sweep_stages ? &m.bwd_t_serial : &m.bwd_serial };
+  for (const LevelSchedule* s : order)
     for (int32_t it = 0; it < s->n_items(); ++it)
     {
       double v = x[s->item_target[it]];
@@ -245,12 +248,49 @@ extern "C" int64_t check_group_lists(const micmb_mechanism_desc* desc, int32_t G
     }
   same(c.E.data() + L.v0, x);
 
-  c.CheckGather(c.p.forcing, m.f_start, m.f_rxn, m.f_coef, L.rate, L.v0, [](int) { return 0; });
-  c.CheckGather(c.p.jacobian, m.j_start, m.j_info, m.j_coef, L.w0, 0, [&](int e) { return row_of[e] >= 0; });
-  for (const GroupPhase* ph : { &c.p.forcing, &c.p.jacobian, &c.p.lu, &c.p.solve })
+  const auto plain = [](int) { return 0; };
+  if (sweep_stages == 0)
+    c.CheckGather(c.p.forcing, m.f_start, m.f_rxn, m.f_coef, L.rate, L.v0, plain);
+  else
   {
+    // contributions are numbered reaction by reaction: reactants, then (stage, q, o)
+    std::vector<int32_t> owner;
+    for (int32_t r = 0; r < m.R; ++r)
+    {
+      const int32_t r0 = m.react_start[r], r1 = m.react_start[r + 1];
+      c.bad += c.p.step_start.at(r) != (int32_t)owner.size();
+      owner.insert(owner.end(), m.react_ids.begin() + r0, m.react_ids.begin() + r1);
+      for (int32_t st = 0; st < sweep_stages; ++st)
+        for (int32_t q = r0; q < r1; ++q)
+          for (int32_t o = r0; o < r1; ++o)
+            if (q != o)
+              owner.push_back(m.react_ids[o]);
+    }
+    auto check = [&](const GroupPhase& ph, const std::vector<int32_t>& species, const std::function<int(int)>& element) {
+      std::vector<int32_t> start{ 0 }, src;
+      for (int32_t i = 0; i < m.S; ++i)
+      {
+        for (int32_t x = 0; x < (int32_t)species.size(); ++x)
+          if (species[x] == i)
+          {
+            src.push_back(element(x));
+            c.InRange(src.back());
+            c.bad += src.back() >= m.nnz && src.back() < L.slot;  // neither vectors nor constants
+          }
+        start.push_back((int32_t)src.size());
+      }
+      c.CheckGather(ph, start, src, std::vector<double>(src.size(), 1.0), 0, L.v0, plain);
+    };
+    check(c.p.forcing, m.react_ids, [&](int x) { return L.slot + x; });
+    check(c.p.step, owner, [&](int x) { return x < m.nnz ? x : L.slot + x - m.nnz; });
+  }
+  c.CheckGather(c.p.jacobian, m.j_start, m.j_info, m.j_coef, L.w0, 0, [&](int e) { return row_of[e] >= 0; });
+  for (const GroupPhase* ph : { &c.p.forcing, &c.p.jacobian, &c.p.lu, &c.p.solve, &c.p.step })
+  {
+    if (ph == &c.p.step && sweep_stages == 0)
+      continue;
     // one unit past the last warp's is fetched
-    const bool gather = ph == &c.p.forcing || ph == &c.p.jacobian;
+    const bool gather = ph != &c.p.lu && ph != &c.p.solve;
     const size_t units = ph->warp_start.back() + 1, lanes = units * (32 / G);
     c.bad += ph->ctrl.size() != units || ph->item.size() != 4 * lanes || ph->row.size() != (gather ? 8 : 16) * lanes ||
              ph->coef.size() != (gather ? 16 * lanes : 0);

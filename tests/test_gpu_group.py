@@ -10,6 +10,7 @@ import pytest
 from micm_b200 import Solver, micm_bench, synthetic
 from micm_b200 import solver as sv
 from micm_b200._native import check, lib
+from micm_b200.mechanism import Mechanism, arrhenius
 from gpu_helpers import download_cols, make_state, upload_cols
 
 pytestmark = pytest.mark.gpu
@@ -145,3 +146,41 @@ def test_single_stages_do_not_depend_on_the_block_shape(cuda_device, name, n, L)
     few = stages(slice(n - 100, n))
     for a, b in zip(many, few):
         np.testing.assert_array_equal(a[n - 100:].view(np.int64), np.ascontiguousarray(b).view(np.int64))
+
+
+def _reactant_orders():
+    """One to three reactants, repeated ones among them, and a source."""
+    m = Mechanism(species=["A", "B", "C", "D"], reactions=[], name="orders")
+    m.add(arrhenius(A=0.3), [0, 0], [(1, 2.0), (1, 0.5)])
+    m.add(arrhenius(A=0.2), [1, 1, 2], [(0, 1.0), (2, 1.0)])
+    m.add(arrhenius(A=0.1), [2, 3, 0], [(2, 1.0)])
+    m.add(arrhenius(A=0.01), [], [(3, 1.0)])
+    m.add(arrhenius(A=0.05), [3], [(0, 1.0)])
+    return m
+
+
+CASES["orders"] = (_reactant_orders, lambda m, n: synthetic.cell_inputs(m, n, 8, log10_conc=(-1.0, 0.3)), 30.0)
+
+
+# The backward sweep on cell groups needs the stored stages; a limit that has room
+# for the states alone makes the one-cell-per-thread kernel recompute them.
+@pytest.mark.parametrize("name,n,L,stages", [("readme", 5003, 32, 2), ("chapman", 149, 100, 3), ("orders", 1, 1, 4),
+                                             ("orders", 777, 8, 60), ("c60", 299, 7, 40), ("c60", 1201, 32, 3),
+                                             ("c210", 149, 128, 4)])
+def test_backward_sweep_equals_thread_kernel(cuda_device, name, n, L, stages):
+    make, inputs, dt = CASES[name]
+    mech = make()
+    inp = inputs(mech, n)
+    ybar = np.random.default_rng(2).normal(size=(n, mech.n_species))
+    got = []
+    for recompute in (True, False):
+        solver = Solver(mech, stages, vector_length=L)
+        if recompute:
+            solver.set_adjoint_memory_limit(-(-n // L) * L * 400 * (mech.n_species + 1) * 8 + 100)
+        st = make_state(solver, inp)
+        solver.update_state_parameters(st)
+        g0, gk, res = solver.solve_adjoint(dt, st, ybar, max_checkpoints=400)
+        assert res.converged
+        got.append((g0.copy(), gk.copy()))
+    np.testing.assert_array_equal(got[1][0], got[0][0])
+    np.testing.assert_array_equal(got[1][1], got[0][1])

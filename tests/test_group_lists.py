@@ -40,7 +40,7 @@ def check(tmp_path_factory):
                     os.path.join(ROOT, "tests", "cpp", "group_lists.cpp"), os.path.join(CSRC, "group.cpp"),
                     os.path.join(CSRC, "mechanism.cpp")], check=True)
     f = C.CDLL(so).check_group_lists
-    f.restype, f.argtypes = C.c_int64, [C.POINTER(MechanismDesc), C.c_int32, C.c_int32]
+    f.restype, f.argtypes = C.c_int64, [C.POINTER(MechanismDesc)] + 3 * [C.c_int32]
     return f
 
 
@@ -48,4 +48,12 @@ def check(tmp_path_factory):
 @pytest.mark.parametrize("G,W", [(1, 1), (1, 8), (2, 4), (4, 2), (8, 8), (16, 4), (32, 1), (32, 8)])
 def test_work_lists_equal_the_serial_schedules(check, name, G, W):
     desc = DescHolder(MECHS[name]().flat())
-    assert check(C.byref(desc.desc), G, W) == 0
+    assert check(C.byref(desc.desc), G, W, 0) == 0
+
+
+# the adjoint's backward sweep: transposed factors, contributions of 2 to 6 stages
+@pytest.mark.parametrize("name", sorted(MECHS))
+@pytest.mark.parametrize("G,W,stages", [(1, 8, 3), (4, 2, 6), (8, 8, 4), (32, 1, 2)])
+def test_backward_sweep_work_lists(check, name, G, W, stages):
+    desc = DescHolder(MECHS[name]().flat())
+    assert check(C.byref(desc.desc), G, W, stages) == 0
