@@ -54,9 +54,9 @@ namespace micmb
       int32_t sync = kGroupNoSync;
     };
 
-    // The chunks of one level, longest first within each kind, as units; a long
-    // chunk's units stay together.
-    std::vector<std::vector<Step>> Pack(const std::vector<Chunk>& chunks)
+    // The chunks of one level, longest first within each kind, as units of at most
+    // `limit` chunks; a long chunk's units stay together.
+    std::vector<std::vector<Step>> Pack(const std::vector<Chunk>& chunks, size_t limit = 4)
     {
       std::vector<std::vector<Step>> out;
       for (size_t i = 0; i < chunks.size();)
@@ -78,7 +78,7 @@ namespace micmb
           continue;
         }
         Step st;
-        const size_t most = T > kGroupTerms / 4 ? 2 : 4;
+        const size_t most = std::min<size_t>(limit, T > kGroupTerms / 4 ? 2 : 4);
         for (; i < chunks.size() && st.chunks.size() < most && chunks[i].kind == kind; ++i)
           st.chunks.push_back(chunks[i]);
         out.back().push_back(std::move(st));
@@ -251,9 +251,12 @@ namespace micmb
       return levels;
     }
 
-    // A level with at most this many units runs on the first warp alone, with
-    // warp synchronisation: a block barrier costs more than a second unit.
-    constexpr size_t kNarrowUnits = 2;
+    // A level with at most this many units runs on the first warp alone, with warp
+    // synchronisation.  A second unit costs about as much as a block barrier:
+    // measured with 1 / 2 / 3 / 4 units, ms: TS1 10,000 cells 62.0 / 64.1 / 67.7 /
+    // 69.2, 210 species 65,536 cells 453 / 460 / 486 / 513, 600 species 700 cells
+    // 100.5 / 99.3 / - / 101.9; with none, 64.2, 477, 104.8.
+    constexpr size_t kNarrowUnits = 1;
 
     // Unit lists of one or more level schedules run one after the other.
     struct LevelLists
@@ -284,7 +287,16 @@ namespace micmb
           if (units.empty())
             continue;
           kept.push_back(std::move(units));
-          std::vector<std::vector<Step>> packed = Pack(Cut(kept.back(), ipw));
+          // as few chunks per unit as give every warp one unit: a warp's time goes with
+          // its unit's terms (TS1, 10,000 cells: 62.0 -> 59.9 ms)
+          const std::vector<Chunk> chunks = Cut(kept.back(), ipw);
+          std::vector<std::vector<Step>> packed;
+          for (size_t limit = 1; limit <= 4; limit *= 2)
+          {
+            packed = Pack(chunks, limit);
+            if (packed.size() <= lists.warp.size())
+              break;
+          }
           size_t n_units = 0;
           for (const auto& steps : packed)
             n_units += steps.size();
