@@ -84,7 +84,7 @@ namespace micmb
     d.inv_order = 1 / p.estimator_of_local_order;
     // safety / error^(1 / order) decreases with the error: where it is past a
     // clamp by more than any rounding, the clamp is the step-size factor and the
-    // power (8,500 cycles in double-double) need not be formed
+    // power (a logarithm and two exps in double-double) need not be formed
     d.error_lo = -1.0;
     d.error_hi = INFINITY;
     const double order = p.estimator_of_local_order;
