@@ -256,7 +256,12 @@ namespace micmb
   {
     const auto& m = *s.mech;
     const int64_t n = st.n_cells;
-    if (n < 1 || !GroupFasterThanStages(s, n))
+    // With one step size every cell takes every attempt, and the per-stage kernels
+    // have no lanes that wait for others': they are the faster form at large counts
+    // (210 species, 1,048,576 cells, ms per attempt: 95 against 129), the cell groups
+    // far below the count that fills the GPU with threads (TS1, 10,000 cells: 641 ->
+    // 70 ms).  The line lies at half of the fused kernels'.
+    if (n < 1 || !GroupFaster(s, n) || !GroupFaster(s, 2 * n))
       return false;
     if (n == 1 && !st.gx_fn)
     {
