@@ -9,6 +9,8 @@
 #include "runtime.hpp"
 
 #include <algorithm>
+#include <mutex>
+#include <set>
 
 namespace micmb
 {
@@ -253,6 +255,20 @@ namespace micmb
     }
   }  // namespace
 
+  void AllowSharedMemory(const micmb_solver& s, const void* kernel)
+  {
+    static std::mutex mutex;
+    static std::set<std::pair<const void*, int>> raised;
+    std::lock_guard<std::mutex> lock(mutex);
+    if (raised.count({ kernel, s.device }))
+      return;
+    cudaFuncAttributes a{};
+    MICMB_CUDA(cudaFuncGetAttributes(&a, kernel));
+    MICMB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)(s.smem_optin - a.sharedSizeBytes)));
+    raised.insert({ kernel, s.device });
+  }
+
   size_t FusedSharedBytes(const micmb_solver& s, bool lu_in_shared)
   {
     const auto& m = *s.mech;
@@ -384,7 +400,7 @@ namespace micmb
     const size_t smem = (size_t)W.per_warp * sizeof(double) * warps;
     const int threads = warps * kWarp;
     auto kernel = lu_shared ? k_fused<true> : k_fused<false>;
-    MICMB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    AllowSharedMemory(s, reinterpret_cast<const void*>(kernel));
     int per_sm = 0;
     MICMB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
     if (per_sm < 1)

@@ -364,7 +364,7 @@ namespace micmb
     // the kernels' static shared memory: at most 96 bytes per cell and a few words
     if (smem + 96 * (size_t)choice.G + 1024 > s.smem_optin)
       return 0;
-    MICMB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    AllowSharedMemory(s, kernel);
     int per_sm = 0;
     MICMB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * choice.W, smem));
     return per_sm;

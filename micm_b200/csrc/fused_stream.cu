@@ -494,7 +494,7 @@ namespace micmb
                 int64_t grid)
     {
       auto kernel = k_fused_stream<W>;
-      MICMB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LY.total_bytes));
+      AllowSharedMemory(s, reinterpret_cast<const void*>(kernel));
       const StepBounds B = step_bounds(s.params, st.dt_for_launch);
       kernel<<<(unsigned)grid, (W + 1) * 32, LY.total_bytes, st.stream>>>(s.dev, s.params, B, A, SA, LY);
       MICMB_CUDA(cudaGetLastError());

@@ -228,6 +228,10 @@ namespace micmb
   void LaunchDecompose(micmb_solver& s, micmb_state& st);
   void LaunchLinearSolve(micmb_solver& s, micmb_state& st);
   void NormalizedError(micmb_solver& s, micmb_state& st, double* global_out, double* per_cell_out);
+  // Lets a kernel use all the dynamic shared memory that the device has for it.  The
+  // limit belongs to the kernel, which the solvers of all threads share: it is raised
+  // once per device and never lowered to one solver's size.
+  void AllowSharedMemory(const micmb_solver& s, const void* kernel);
   size_t FusedSharedBytes(const micmb_solver& s, bool lu_in_shared);
   // streamed warp-specialised variant; returns false when it does not apply
   bool SolveFusedStream(micmb_solver& s, micmb_state& st, double dt, const FusedArgs& A);
