@@ -553,6 +553,14 @@ namespace micmb
       count_attempt(cc, P);
       const int res = ctl_after_error(cc, P, b, error);
       *last_accept = (res == 1);
+      // a solve ends with the attempt that completes it, as on the cell-group kernels: the
+      // ranks of a job may run either, and have to make the same number of exchanges
+      CellCtl next = cc;
+      if (res == 1 && !ctl_begin_step(next, P, b))
+      {
+        cc.state = next.state;
+        cc.new_step = 0;
+      }
       a.status[0] = cc.state;
       a.ctl[0] = cc;
     }
