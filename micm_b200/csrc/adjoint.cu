@@ -961,15 +961,14 @@ namespace micmb
       {
         const int64_t blocks = std::min<int64_t>((int64_t)group_blocks * s.sm_count, (n + choice.G - 1) / choice.G);
         const int64_t slot = ((int64_t)m.S * (2 + 3 * s.params.stages) + 2 * (int64_t)m.R) * choice.G;
-        EnsureGroupWorkspace(st, blocks * slot);
+        EnsureWorkspace(st, st.group_ws, blocks * slot);
         group<<<(unsigned)blocks, 32 * choice.W, GroupSharedBytes(s, choice), st.stream>>>(
             s.dev, GroupTablesFor(s, choice).dev, s.params, A, st.group_ws.as<double>(), slot);
         MICMB_CUDA(cudaGetLastError());
         return;
       }
       const int64_t doubles = grid * 128 * (int64_t)T.per_slot;
-      if (!st.thread_ws.p || st.thread_ws.bytes < (size_t)doubles * sizeof(double))
-        st.thread_ws = DeviceMemory((size_t)doubles * sizeof(double));
+      EnsureWorkspace(st, st.thread_ws, doubles);
       kernel<<<(unsigned)grid, 128, 0, st.stream>>>(s.dev, s.params, A, T, st.thread_ws.as<double>());
       MICMB_CUDA(cudaGetLastError());
     }

@@ -597,7 +597,7 @@ namespace micmb
       const int per_sm = GroupBlocksPerSm(s, kernel, choice);
       gg.blocks = std::min<int64_t>((int64_t)per_sm * s.sm_count, (n + choice.G - 1) / choice.G);
       gg.slot = doubles_per_cell * choice.G;
-      EnsureGroupWorkspace(st, gg.blocks * gg.slot);
+      EnsureWorkspace(st, st.group_ws, gg.blocks * gg.slot);
       return gg;
     }
 
@@ -872,8 +872,7 @@ namespace micmb
         int64_t grid = (int64_t)per_sm * s.sm_count;
         grid = std::max<int64_t>(1, std::min<int64_t>(grid, (n + kThreadsPerBlock - 1) / kThreadsPerBlock));
         const int64_t doubles = grid * kThreadsPerBlock * (int64_t)T.per_slot;
-        if (!st.thread_ws.p || st.thread_ws.bytes < (size_t)doubles * sizeof(double))
-          st.thread_ws = DeviceMemory((size_t)doubles * sizeof(double));
+        EnsureWorkspace(st, st.thread_ws, doubles);
         k_backward_euler_thread<<<(unsigned)grid, kThreadsPerBlock, 0, stream>>>(s.dev, P, dt, A,
                                                                                   st.thread_ws.as<double>(), T);
         MICMB_CUDA(cudaGetLastError());

@@ -55,6 +55,24 @@ namespace micmb
     return *this;
   }
 
+  void DropCapturedSolve(micmb_state& st)
+  {
+    if (!st.graph_exec)
+      return;
+    MICMB_CUDA(cudaGraphExecDestroy(st.graph_exec));
+    st.graph_exec = nullptr;
+  }
+
+  void EnsureWorkspace(micmb_state& st, DeviceMemory& ws, int64_t doubles)
+  {
+    const size_t bytes = sizeof(double) * (size_t)doubles;
+    if (ws.p && ws.bytes >= bytes)
+      return;
+    DropCapturedSolve(st);
+    ws = DeviceMemory();  // before the new one, so that both need not fit
+    ws = DeviceMemory(bytes);
+  }
+
   DevParams ToDevParams(const micmb_rosenbrock_params& p)
   {
     if (p.stages < 1 || p.stages > 6)
@@ -1067,11 +1085,7 @@ extern "C"
         st.accepted = DeviceMemory(sizeof(int32_t) * std::max<int64_t>(n, 1));
       // per-thread working sets do not shrink with the chunk: size them first
       const int64_t ws = std::max(FusedThreadWorkspaceDoubles(*solver, n), AdjointThreadWorkspaceDoubles(*solver, n));
-      if (!st.thread_ws.p || st.thread_ws.bytes < (size_t)ws * sizeof(double))
-      {
-        st.thread_ws = DeviceMemory();
-        st.thread_ws = DeviceMemory((size_t)ws * sizeof(double));
-      }
+      EnsureWorkspace(st, st.thread_ws, ws);
 
       // Checkpoints take max_checkpoints * (S + 1) doubles per cell, the stored
       // stage vectors max_checkpoints * stages * S more.  Cells are solved and

@@ -370,19 +370,6 @@ namespace micmb
     return per_sm;
   }
 
-  void EnsureGroupWorkspace(micmb_state& st, int64_t doubles)
-  {
-    if (st.group_ws.bytes >= sizeof(double) * (size_t)doubles)
-      return;
-    // a captured solve holds the old workspace's address
-    if (st.graph_exec)
-    {
-      MICMB_CUDA(cudaGraphExecDestroy(st.graph_exec));
-      st.graph_exec = nullptr;
-    }
-    st.group_ws = DeviceMemory(sizeof(double) * (size_t)doubles);
-  }
-
   bool GroupVariantApplies(const micmb_solver& s, int64_t n_cells)
   {
     // the register-blocked schedules, asked for by the environment, are the
@@ -432,7 +419,7 @@ namespace micmb
     const int64_t grid =
         std::max<int64_t>(1, std::min<int64_t>((int64_t)per_sm * s.sm_count, (A.n_cells + choice.G - 1) / choice.G));
     const int64_t slot = (GroupVectorDoubles(s.mech->S, s.params.stages) + s.mech->R) * choice.G;
-    EnsureGroupWorkspace(st, grid * slot);
+    EnsureWorkspace(st, st.group_ws, grid * slot);
     kernel<<<(unsigned)grid, 32 * choice.W, GroupSharedBytes(s, choice), st.stream>>>(
         t.dev, s.params, step_bounds(s.params, dt), A, st.group_ws.as<double>(), slot);
     MICMB_CUDA(cudaGetLastError());

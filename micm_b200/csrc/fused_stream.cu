@@ -551,6 +551,7 @@ namespace micmb
     if (order != st.attempt_order_host)
     {
       // uploaded once per tableau, so repeated launches (and graph captures) copy nothing
+      DropCapturedSolve(st);
       MICMB_CUDA(cudaStreamSynchronize(st.stream));  // no earlier launch still reads the old order
       if (st.attempt_order.bytes < order.size() * sizeof(int32_t))
         st.attempt_order = DeviceMemory(order.size() * sizeof(int32_t));
@@ -579,11 +580,7 @@ namespace micmb
     {
       const int64_t slots_needed = grid * W;
       const int64_t stride = ((int64_t)m.nnz + 2 + 31) & ~31ll;
-      if (st.lu_slot_count < slots_needed * stride || !st.lu_slots.p)
-      {
-        st.lu_slots = DeviceMemory(sizeof(double) * (size_t)(slots_needed * stride));
-        st.lu_slot_count = slots_needed * stride;
-      }
+      EnsureWorkspace(st, st.lu_slots, slots_needed * stride);
       A.lu_global = st.lu_slots.as<double>();
       A.lu_slot_stride = stride;
     }

@@ -416,8 +416,7 @@ namespace micmb
     int64_t grid = (int64_t)per_sm * s.sm_count;
     grid = std::max<int64_t>(1, std::min<int64_t>(grid, (A_in.n_cells + kThreadsPerBlock - 1) / kThreadsPerBlock));
     const int64_t doubles = grid * kThreadsPerBlock * (int64_t)T.per_slot;
-    if (!st.thread_ws.p || st.thread_ws.bytes < (size_t)doubles * sizeof(double))
-      st.thread_ws = DeviceMemory((size_t)doubles * sizeof(double));
+    EnsureWorkspace(st, st.thread_ws, doubles);
     const StepBounds B = step_bounds(s.params, dt);
     kernel<<<(unsigned)grid, kThreadsPerBlock, 0, st.stream>>>(s.dev, s.params, B, A_in, st.thread_ws.as<double>(),
                                                                T);

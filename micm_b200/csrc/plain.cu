@@ -718,7 +718,9 @@ namespace micmb
     if (!st.ctl.p)
     {
       st.ctl = DeviceMemory(sizeof(CellCtl) * std::max<int64_t>(st.n_cells, 1));
-      st.status = DeviceMemory(sizeof(int32_t) * std::max<int64_t>(st.n_cells, 1));
+      // fused solves, captured ones among them, write their statuses there too
+      if (!st.status.p)
+        st.status = DeviceMemory(sizeof(int32_t) * std::max<int64_t>(st.n_cells, 1));
     }
   }
 

@@ -285,7 +285,7 @@ namespace micmb
     const GroupTables& t = GroupTablesFor(s, choice);
     const int64_t grid = std::min<int64_t>((int64_t)per_sm * s.sm_count, (n + choice.G - 1) / choice.G);
     const int64_t slot = GroupVectorDoubles(m.S, s.params.stages) * choice.G;
-    EnsureGroupWorkspace(st, grid * slot);
+    EnsureWorkspace(st, st.group_ws, grid * slot);
     const unsigned n_blk = Blocks(n);
     if (!st.group_ynew.p)
       st.group_ynew = DeviceMemory(st.dense_bytes(m.S));

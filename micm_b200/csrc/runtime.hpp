@@ -146,7 +146,6 @@ struct micmb_state
   int32_t* host_counters = nullptr;  // pinned
   // fused path
   micmb::DeviceMemory lu_slots;
-  int64_t lu_slot_count = 0;  // doubles allocated in lu_slots
   micmb::DeviceMemory group_ws;   // cell-group kernels: the cells' vectors outside shared memory
   micmb::DeviceMemory group_ynew, group_err, group_ctl;  // plain method on them: Ynew, error sums, control
   micmb::DeviceMemory thread_ws;  // one-cell-per-thread variant: per-thread working sets
@@ -247,8 +246,11 @@ namespace micmb
   int GroupBlocksPerSm(const micmb_solver& s, const void* kernel, const GroupChoice& choice);
   bool GroupVariantApplies(const micmb_solver& s, int64_t n_cells);
   int32_t GroupCellsPerSm(const micmb_solver& s);
-  // st.group_ws of at least that many doubles
-  void EnsureGroupWorkspace(micmb_state& st, int64_t doubles);
+  // Destroys the state's captured solve, which holds the addresses of the buffers it
+  // was captured with: to be called before one of them is replaced.
+  void DropCapturedSolve(micmb_state& st);
+  // a state's workspace of at least that many doubles
+  void EnsureWorkspace(micmb_state& st, DeviceMemory& ws, int64_t doubles);
   bool GroupFaster(const micmb_solver& s, int64_t n_cells);  // than the one-cell-per-thread kernel
   bool GroupFasterThanStages(const micmb_solver& s, int64_t n_cells);  // than the plain per-stage kernels
   void SolveFusedGroup(micmb_solver& s, micmb_state& st, const FusedArgs& A, double dt);
