@@ -4,6 +4,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 #include <fstream>
 #include <sstream>
 #include <string>
@@ -221,7 +222,8 @@ extern "C"
 
   // n_repeats x (UpdateStateParameters + fused Solve): the first repeat runs
   // eagerly (allocating the working set), is then captured once into a CUDA
-  // graph for this state, dt and configuration, and the graph is replayed.
+  // graph for this state, dt, tolerance, parameters and configuration, and the
+  // graph is replayed.
   int micmb_solve_graph(micmb_solver* solver, micmb_state* state, double dt, int32_t n_repeats)
   {
     return GuardX([&] {
@@ -231,14 +233,12 @@ extern "C"
       MICMB_CUDA(cudaSetDevice(solver->device));
       micmb_state& st = *state;
       int32_t done = 0;
-      const bool reuse = st.graph_exec && st.graph_dt == dt && SameConfig(st.graph_config, solver->fused);
+      const bool reuse = st.graph_exec && st.graph_dt == dt && st.graph_rtol == st.rtol &&
+                         SameConfig(st.graph_config, solver->fused) &&
+                         std::memcmp(&st.graph_params, &solver->host_params, sizeof(st.graph_params)) == 0;
       if (!reuse && n_repeats > 0)
       {
-        if (st.graph_exec)
-        {
-          MICMB_CUDA(cudaGraphExecDestroy(st.graph_exec));
-          st.graph_exec = nullptr;
-        }
+        DropCapturedSolve(st);
         EnqueueStep(*solver, st, dt);
         CheckFusedError(st);
         ++done;
@@ -260,6 +260,8 @@ extern "C"
         cudaGraphDestroy(graph);
         MICMB_CUDA(ie);
         st.graph_dt = dt;
+        st.graph_rtol = st.rtol;
+        st.graph_params = solver->host_params;
         st.graph_config = solver->fused;
       }
       for (; done < n_repeats; ++done)

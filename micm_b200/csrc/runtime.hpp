@@ -154,8 +154,10 @@ struct micmb_state
   int64_t solve_limit = 0;                  // fused solves: only the first solve_limit cells (0 = all)
   // CUDA graph of UpdateStateParameters + fused Solve (micmb_solve_graph)
   cudaGraphExec_t graph_exec = nullptr;
-  double graph_dt = 0.0;
+  // what the capture took from outside the device buffers
+  double graph_dt = 0.0, graph_rtol = 0.0;
   micmb_fused_config graph_config{};
+  micmb_rosenbrock_params graph_params{};
   // adjoint working set (allocated on first use)
   micmb::DeviceMemory adj_y0, adj_ybar, adj_ckpt_y, adj_ckpt_h, adj_ckpt_k, adj_kbar_cells, adj_kbar;
   micmb::DeviceMemory be_ctl;     // Backward Euler global control block

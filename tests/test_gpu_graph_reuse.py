@@ -1,6 +1,8 @@
 """A captured solve (micmb_solve_graph) between other calls on the same state:
 calls that replace a buffer the capture holds, and settings that it was captured
 with."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -50,6 +52,36 @@ def test_captured_solve_after_other_calls(cuda_device, config, between):
                     solver.solve(30.0, st, method="fused", step_control="per_cell")
         steps(2)
         between(solver, st)
+        steps(2)
+        st.sync_outputs_to_host()
+        outs.append(st.concentrations())
+    np.testing.assert_array_equal(outs[1], outs[0])
+
+
+@pytest.mark.parametrize("what", ["tolerance", "params"])
+def test_captured_solve_follows_changed_settings(cuda_device, what):
+    """The relative tolerance and the solver's parameters are part of a capture."""
+    cfg = synthetic.CONFIGS["c60_adjoint"]
+    mech = cfg["mech"]()
+    inputs = synthetic.cell_inputs(mech, 64, 18)
+    outs = []
+    for graph in (False, True):
+        solver = Solver(mech, cfg["stages"], vector_length=32)
+        st = make_state(solver, inputs)
+
+        def steps(n):
+            if graph:
+                solver.solve_graph(600.0, st, n)
+            else:
+                for _ in range(n):
+                    solver.update_state_parameters(st)
+                    solver.solve(600.0, st, method="fused", step_control="per_cell")
+        steps(2)
+        if what == "tolerance":
+            check(lib().micmb_state_set_relative_tolerance(st.handle, 1.0e-4))
+        else:
+            solver.params.safety_factor = 0.7
+            check(lib().micmb_solver_set_params(solver.handle, C.byref(solver.params)))
         steps(2)
         st.sync_outputs_to_host()
         outs.append(st.concentrations())
