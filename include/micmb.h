@@ -325,9 +325,9 @@ typedef struct micmb_fused_config {
                               the 32-register one (every warp slot of the SM) */
   int32_t ring_slots;      /* streamed variant: shared-memory slots for table blocks (0 = 4) */
   int32_t variant;         /* 0 cell groups (a block advances several cells in lockstep, working
-                              sets in shared memory), or streamed (TMA-fed, warp-specialised)
-                              where a reaction has more than three reactants; 1 direct (warp per
-                              cell); 2 one cell per thread (working sets in global memory), or
+                              sets in shared memory); streamed (TMA-fed, warp-specialised) where
+                              cells_per_cta, ctas_per_sm or ring_slots asks for it or a reaction
+                              has more than three reactants; 1 direct (warp per cell); 2 one cell per thread (working sets in global memory), or
                               cell groups for fewer cells than fill the GPU, unless ctas_per_sm
                               asks for a build.  Results do not depend on it. */
 } micmb_fused_config;

@@ -113,6 +113,7 @@ extern "C"
       }
       micmb_state& st = *state;
       const micmb_fused_config candidates[] = {
+        { 0, 1, 0, 0, 0 },                     // cell groups
         { 0, 1, 0, 2, 0 }, { 0, 1, 0, 4, 0 },  // streamed, LU in shared memory
         { 0, 0, 0, 2, 0 }, { 0, 0, 0, 4, 0 },  // streamed, LU in global slots, as many cells as fit
         { 6, 0, 0, 4, 0 }, { 4, 0, 0, 4, 0 },  // streamed, fewer cells per CTA
@@ -169,9 +170,11 @@ extern "C"
         const bool has_stream = solver->dev.has_warp && solver->stream_blocks.p;
         for (const auto& c : candidates)
         {
-          const bool group = c.variant == 0 && GroupVariantApplies(*solver, trial_cells(c));
-          // the cell-group kernel takes none of the streamed kernel's settings: one trial
-          if ((c.variant == 0 && !(group ? &c == candidates : has_stream)) ||
+          // the streamed kernel only where there are no cell groups: 60 species, 800,000
+          // cells 2,250 against 774 ms, Chapman, 1,000,000 246 against 17, 210 species, one
+          // cell 12.9 against 6.6
+          const bool groups = GroupVariantApplies(*solver, trial_cells(c));
+          if ((c.variant == 0 && (c.ring_slots == 0 ? !groups : groups || !has_stream)) ||
               (c.variant == 1 && !solver->dev.has_warp))
             continue;
           const double r = rate_of(c, trial_cells(c), 2);

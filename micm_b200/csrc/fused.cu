@@ -377,8 +377,11 @@ namespace micmb
     const int64_t n = (adj && adj->n_cells > 0)
                           ? adj->n_cells
                           : (st.solve_limit > 0 ? std::min<int64_t>(st.solve_limit, st.n_cells) : st.n_cells);
-    // variant 2 without a chosen build: the thread kernel where it is the faster one
-    const bool group = n > 0 && ((s.fused.variant == 0 && GroupVariantApplies(s, n)) ||
+    // variant 0 with a setting of the streamed kernel asks for that one; variant 2 without
+    // a chosen build: the thread kernel where it is the faster one
+    const bool asks_streamed = s.fused.cells_per_cta > 0 || s.fused.ctas_per_sm > 0 || s.fused.ring_slots > 0;
+    const bool group = n > 0 && ((s.fused.variant == 0 && !(asks_streamed && StreamVariantApplies(s)) &&
+                                  GroupVariantApplies(s, n)) ||
                                  (s.fused.variant == 2 && s.fused.ctas_per_sm == 0 && GroupFaster(s, n)));
     if (group)
     {

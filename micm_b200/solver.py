@@ -166,8 +166,9 @@ class Solver:
         check(lib().micmb_solver_set_rate_scale(self.handle, _f64(scale)))
 
     def set_fused_config(self, cells_per_cta=0, lu_in_shared=1, ctas_per_sm=0, ring_slots=0, variant=0):
-        """variant 0: TMA-streamed warp-specialised kernel; 1: direct kernel (warp per cell);
-        2: one cell per thread, working sets in global memory."""
+        """variant 0: cell groups, or with cells_per_cta, ctas_per_sm or ring_slots set the
+        TMA-streamed warp-specialised kernel; 1: direct kernel (warp per cell); 2: one cell per
+        thread, working sets in global memory."""
         cfg = FusedConfig(int(cells_per_cta), int(lu_in_shared), int(ctas_per_sm), int(ring_slots), int(variant))
         check(lib().micmb_solver_set_fused_config(self.handle, C.byref(cfg)))
 
