@@ -81,6 +81,10 @@ namespace micmb
         throw Error(MICMB_ERR_TIMEOUT, "fused kernel: a pipeline wait timed out");
     }
 
+    // micmb_fused_config.ctas_per_sm of the 32-register thread build: all of the SM's
+    // blocks, asked for as such (0 leaves small counts to the cell groups)
+    constexpr int32_t kFullBuild = 16;
+
     bool SameConfig(const micmb_fused_config& a, const micmb_fused_config& b)
     {
       return a.cells_per_cta == b.cells_per_cta && a.lu_in_shared == b.lu_in_shared &&
@@ -118,7 +122,7 @@ extern "C"
         { 0, 0, 0, 2, 0 }, { 0, 0, 0, 4, 0 },  // streamed, LU in global slots, as many cells as fit
         { 6, 0, 0, 4, 0 }, { 4, 0, 0, 4, 0 },  // streamed, fewer cells per CTA
         { 0, 1, 0, 0, 1 }, { 0, 0, 0, 0, 1 },  // direct
-        { 0, 0, 0, 0, 2 }, { 0, 0, 12, 0, 2 },  // one cell per thread: 32-, 40-, 64- and 96-register builds
+        { 0, 0, kFullBuild, 0, 2 }, { 0, 0, 12, 0, 2 },  // one cell per thread: 32-, 40-, 64- and 96-register builds
         { 0, 0, 8, 0, 2 }, { 0, 0, 5, 0, 2 },
       };
       // tune each candidate on enough cells to fill every SM a few times over:
@@ -212,6 +216,9 @@ extern "C"
         throw;
       }
       st.solve_limit = 0;
+      // the build that 0 stands for, unless 0 would mean the cell groups here
+      if (best.variant == 2 && best.ctas_per_sm == kFullBuild && !GroupFaster(*solver, st.n_cells))
+        best.ctas_per_sm = 0;
       MICMB_CUDA(cudaMemcpyAsync(st.variables.p, saved.p, st.variables.bytes, cudaMemcpyDeviceToDevice, st.stream));
       MICMB_CUDA(cudaStreamSynchronize(st.stream));
       cudaEventDestroy(e0);
