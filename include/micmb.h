@@ -335,7 +335,8 @@ int micmb_solver_set_fused_config(micmb_solver* solver, const micmb_fused_config
 int micmb_solver_get_fused_config(micmb_solver* solver, micmb_fused_config* config);
 /* Time candidate fused configurations on this state (its current inputs are
  * preserved) and keep the fastest; the choice is cached in `cache_path`
- * (may be NULL) under the mechanism hash. */
+ * (may be NULL) under the mechanism hash, the tableau, the GPU and whether the
+ * state has more cells than the cell groups are best for. */
 int micmb_autotune(micmb_solver* solver, micmb_state* state, double dt, const char* cache_path,
                    micmb_fused_config* chosen);
 

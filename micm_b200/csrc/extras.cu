@@ -26,12 +26,21 @@ namespace micmb
         throw Error(MICMB_ERR_INVALID_ARGUMENT, what);
     }
 
-    // cache key: tables, tableau and the GPU (SM count, shared memory)
-    std::string TuneKey(const micmb_solver& s)
+    // What the configurations stand for: raised when one of them means another kernel,
+    // so that entries of earlier builds are not taken (1, without a tag: variant 0 was
+    // the streamed kernel).
+    constexpr int kTuneVersion = 2;
+
+    // Cache key: tables, tableau, the GPU (SM count, shared memory), and whether the
+    // state has more cells than the cell groups are best for -- the one choice that
+    // depends on the count most (TS1, 1,000,000 cells: 5,806 ms on the groups that win
+    // at small counts, 4,531 on the thread kernel).
+    std::string TuneKey(const micmb_solver& s, int64_t n_cells)
     {
+      const bool few = GroupApplies(*s.mech) ? GroupFaster(s, n_cells) : n_cells <= (int64_t)s.sm_count * 2048;
       char buf[128];
-      std::snprintf(buf, sizeof(buf), "%016llx:%d:%d:%zu", (unsigned long long)s.mech->hash, s.params.stages,
-                    s.sm_count, s.smem_optin);
+      std::snprintf(buf, sizeof(buf), "%016llx:%d:%d:%zu:v%d:%s", (unsigned long long)s.mech->hash, s.params.stages,
+                    s.sm_count, s.smem_optin, kTuneVersion, few ? "few" : "many");
       return buf;
     }
 
@@ -106,7 +115,7 @@ extern "C"
       NeedX(solver && state && state->solver == solver, "state does not belong to this solver");
       NeedX(dt > 0 && std::isfinite(dt), "time step must be positive and finite");
       MICMB_CUDA(cudaSetDevice(solver->device));
-      const std::string key = TuneKey(*solver);
+      const std::string key = TuneKey(*solver, state->n_cells);
       micmb_fused_config best{};
       if (ReadCache(cache_path, key, best))
       {

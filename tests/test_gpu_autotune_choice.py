@@ -1,7 +1,6 @@
 """What the tuner tries, and which states its choice is kept for."""
 import re
 
-import numpy as np
 import pytest
 
 from micm_b200 import Solver, micm_bench
@@ -29,3 +28,25 @@ def test_every_thread_build_is_tried_as_itself(cuda_device, monkeypatch, capfd, 
         assert chosen["variant"] != 2 or chosen["ctas_per_sm"] != 16
     res = solver.solve(micm_bench.DT, st, method="fused", step_control="per_cell")
     assert res.converged
+
+
+def test_choices_of_other_counts_and_builds_are_not_taken(cuda_device, tmp_path):
+    """A choice cached by a state on either side of the hand-over between cell groups
+    and one cell per thread serves that side; entries without the version tag (variant
+    0 was another kernel) serve none."""
+    cache = tmp_path / "tune.txt"
+    _tuned(100, str(cache))
+    small = cache.read_text().splitlines()
+    assert len(small) == 1
+    key = small[0].split()[0]
+    # as an earlier build would have written it
+    cache.write_text(":".join(key.split(":")[:4]) + " 6 0 0 4 0\n")
+    _, _, chosen = _tuned(100, str(cache))
+    assert chosen["cells_per_cta"] != 6 and len(cache.read_text().splitlines()) == 2
+    # a choice for few cells that no large state would make
+    cache.write_text(key + " 0 1 1 0 1\n")
+    _, _, chosen = _tuned(100, str(cache))
+    assert (chosen["variant"], chosen["ctas_per_sm"]) == (1, 1)
+    _, _, chosen = _tuned(400000, str(cache))
+    assert (chosen["variant"], chosen["ctas_per_sm"]) != (1, 1)
+    assert len(cache.read_text().splitlines()) == 2
