@@ -806,7 +806,7 @@ namespace micmb
     {
       if (!GroupFaster(s, n))
         return false;
-      if (s.mech->nnz < 128)
+      if (s.mech->nnz < kTinyNonZeros)
         return n <= (int64_t)s.sm_count * 128;
       return n <= std::min<int64_t>((int64_t)s.sm_count * 1024, 12288 * (int64_t)GroupCellsPerSm(s));
     }

@@ -577,11 +577,24 @@ namespace micmb
       }
     }
 
-    // whether n cells are solved by a cell-group kernel: up to where the
-    // thread-per-cell kernels are faster
+    // Whether n cells are solved by a cell-group kernel: up to where the
+    // thread-per-cell kernels are faster.  Per cell, measured, ms: Chapman 75,000 cells
+    // 0.188 / 0.197, 150,000 0.288 / 0.256; 60 species 303,000 36 / 147; TS1 150,000 548 /
+    // 771; 210 species 262,000 197 / 767; 600 species 32,000 357 / 4,050.
     bool GroupFits(const micmb_solver& s, const void* kernel, const GroupChoice& choice, int64_t n)
     {
-      return n > 0 && GroupFaster(s, n) && GroupBlocksPerSm(s, kernel, choice) > 0;
+      return n > 0 && GroupFaster(s, n) && (s.mech->nnz >= kTinyNonZeros || n <= (int64_t)s.sm_count * 640) &&
+             GroupBlocksPerSm(s, kernel, choice) > 0;
+    }
+
+    // The cells for which an iteration on cell groups takes as long as on one set of
+    // threads, with one step size.  Measured, ms, groups / threads: Chapman 75,000 cells
+    // 0.279 / 0.286, 150,000 0.383 / 0.347; 60 species (32 cells per SM) 150,000 232 / 230,
+    // 225,000 346 / 420; TS1 (8) 75,000 332 / 500, 150,000 655 / 615; 210 species (8)
+    // 130,000 1,241 / 1,191, 196,000 1,896 / 2,187; 600 species (1) 32,000 4,003 / 6,346.
+    int64_t EqualCells(const micmb_solver& s)
+    {
+      return (int64_t)s.sm_count * (s.mech->nnz < kTinyNonZeros ? 640 : (GroupCellsPerSm(s) >= 16 ? 1000 : 840));
     }
 
     // blocks of a cell-group kernel for n cells and the doubles of each
@@ -726,7 +739,9 @@ namespace micmb
       const int64_t n = st.n_cells;
       const GroupChoice choice = ChooseGroup(s, n);
       const GroupIterateKernel iterate = GroupIterateFor(choice.G);
-      const bool group = GroupFits(s, reinterpret_cast<const void*>(iterate), choice, n);
+      const bool group = n > 0 && GroupFaster(s, n) &&
+                         GroupBeatsThreads(s, n, EqualCells(s), reinterpret_cast<const void*>(k_be_iterate), kBlock) &&
+                         GroupBlocksPerSm(s, reinterpret_cast<const void*>(iterate), choice) > 0;
       const DevGroup tables = group ? GroupTablesFor(s, choice).dev : DevGroup{};
       GroupGrid gg;
       if (group)

@@ -267,7 +267,7 @@ namespace micmb
     while (c.G < 32 && n_cells >= (c.G < 8 ? 2 : 4) * (int64_t)c.G * s.sm_count &&
            2 * c.G * per_cell + 1024 <= s.smem_optin)
       c.G *= 2;
-    if (m.nnz < 128)
+    if (m.nnz < kTinyNonZeros)
       return c;
     const int64_t fit = std::max<int64_t>(1, (int64_t)((s.smem_optin + 1024) / (c.G * per_cell + 2048)));
     const int64_t wanted = (n_cells + (int64_t)c.G * s.sm_count - 1) / ((int64_t)c.G * s.sm_count);
@@ -384,24 +384,37 @@ namespace micmb
   // nearly the same time for fewer; the cell-group kernel's time is proportional
   // to the cells from a few thousand on, and inversely to the cells an SM holds.
   // Measured, cell-group against one-cell-per-thread fused kernel, ms: Chapman
-  // 100,000 cells 1.9 / 2.2, 1,000,000 19 / 16; 60 species 262,144 411 / 526,
-  // 1,000,000 1,550 / 1,218; TS1 200,000 1,169 / 1,413, 1,000,000 5,806 / 4,531; 210
-  // species (8 cells per SM) 131,072 933 / 1,478, 262,144 1,859 / 1,896, 524,288
-  // 3,710 / 3,340; 600 species (2 per SM) 20,000 2,532 / 6,182, 100,000 12,593 / 7,442.
+  // 150,000 cells 2.6 / 2.9, 225,000 3.9 / 3.8, 300,000 5.2 / 4.5; 60 species (32 cells
+  // per SM) 300,000 294 / 570, 1,000,000 1,550 / 1,218; TS1 (8 per SM) 260,000 1,388 /
+  // 1,613, 1,000,000 5,806 / 4,531; 210 species (8 per SM) 260,000 1,747 / 1,915,
+  // 524,288 3,710 / 3,340; 600 species (1 per SM) 32,000 4,013 / 6,332, 100,000 12,593 /
+  // 7,442.
   bool GroupFaster(const micmb_solver& s, int64_t n_cells)
   {
     if (!GroupVariantApplies(s, n_cells))
       return false;
-    return n_cells <= std::min<int64_t>((int64_t)s.sm_count * 2048, 32768 * (int64_t)GroupCellsPerSm(s));
+    const int64_t per_sm = s.mech->nnz < kTinyNonZeros ? 1500 : 2048;
+    return n_cells <= std::min<int64_t>(s.sm_count * per_sm, 32768 * (int64_t)GroupCellsPerSm(s));
   }
 
   // The per-stage kernels take 1.3-1.6 times the thread kernel's time, so with
   // eight cells per SM the cell-group kernel is faster at any count (210 species,
-  // 1,048,576 cells: 7.4 s against 8.7 s); with two (600 species) it is up to the
-  // thread kernel's limit.
+  // 1,048,576 cells: 7.4 s against 8.7 s; TS1, 600,000 3.2 against 4.4; Chapman,
+  // 1,000,000 17 ms against 20); with one (600 species) it is up to the thread
+  // kernel's limit.
   bool GroupFasterThanStages(const micmb_solver& s, int64_t n_cells)
   {
     return GroupVariantApplies(s, n_cells) && (GroupCellsPerSm(s) >= 8 || GroupFaster(s, n_cells));
+  }
+
+  bool GroupBeatsThreads(const micmb_solver& s, int64_t n_cells, int64_t equal, const void* kernel, int block)
+  {
+    if (n_cells <= equal)
+      return true;
+    int per_sm = 0;
+    MICMB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, 0));
+    const int64_t set = std::max<int64_t>(1, (int64_t)per_sm * block * s.sm_count);
+    return n_cells <= (n_cells + set - 1) / set * equal;
   }
 
   int32_t GroupCellsPerSm(const micmb_solver& s)

@@ -1038,7 +1038,7 @@ namespace micmb
   void LaunchAddForcing(micmb_solver& s, micmb_state& st)
   {
     EnsurePlainBuffers(st);
-    if (LaunchGroupStage(s, st, GroupStage::kForcing))
+    if (LaunchGroupStage(s, st, GroupStage::kForcing, reinterpret_cast<const void*>(k_add_forcing), kBlock))
       return;
     PlainArgs a = MakeArgs(s, st, 0);
     k_add_forcing<<<Blocks(st.n_cells), kBlock, 0, st.stream>>>(s.dev, a);
@@ -1047,7 +1047,7 @@ namespace micmb
   void LaunchSubtractJacobian(micmb_solver& s, micmb_state& st)
   {
     EnsurePlainBuffers(st);
-    if (LaunchGroupStage(s, st, GroupStage::kJacobian))
+    if (LaunchGroupStage(s, st, GroupStage::kJacobian, reinterpret_cast<const void*>(k_subtract_jacobian), kBlock))
       return;
     PlainArgs a = MakeArgs(s, st, 0);
     k_subtract_jacobian<<<Blocks(st.n_cells), kBlock, 0, st.stream>>>(s.dev, a);
@@ -1064,7 +1064,7 @@ namespace micmb
   void LaunchDecompose(micmb_solver& s, micmb_state& st)
   {
     EnsurePlainBuffers(st);
-    if (LaunchGroupStage(s, st, GroupStage::kLu))
+    if (LaunchGroupStage(s, st, GroupStage::kLu, reinterpret_cast<const void*>(k_decompose_all), kBlock))
       return;
     PlainArgs a = MakeArgs(s, st, 0);
     k_decompose_all<<<Blocks(st.n_cells), kBlock, 0, st.stream>>>(s.dev, a);
@@ -1073,7 +1073,7 @@ namespace micmb
   void LaunchLinearSolve(micmb_solver& s, micmb_state& st)
   {
     EnsurePlainBuffers(st);
-    if (LaunchGroupStage(s, st, GroupStage::kSolve))
+    if (LaunchGroupStage(s, st, GroupStage::kSolve, reinterpret_cast<const void*>(k_linear_solve_all), kBlock))
       return;
     PlainArgs a = MakeArgs(s, st, 0);
     k_linear_solve_all<<<Blocks(st.n_cells), kBlock, 0, st.stream>>>(s.dev, a);

@@ -259,9 +259,15 @@ namespace micmb
     // With one step size every cell takes every attempt, and the per-stage kernels
     // have no lanes that wait for others': they are the faster form at large counts
     // (210 species, 1,048,576 cells, ms per attempt: 95 against 129), the cell groups
-    // far below the count that fills the GPU with threads (TS1, 10,000 cells: 641 ->
-    // 70 ms).  The line lies at half of the fused kernels'.
-    if (n < 1 || !GroupFaster(s, n) || !GroupFaster(s, 2 * n))
+    // below the count that fills the GPU with threads.  Measured, ms, cell groups /
+    // per-stage kernels: Chapman 151,000 cells 2.3 / 3.1; 60 species (32 cells per SM)
+    // 151,000 469 / 621; TS1 (8) 10,000 70 / 641, 130,000 884 / 926; 210 species (8) 98,000
+    // 1,137 / 1,373, 120,000 1,456 / 1,474, 131,000 1,520 / 1,413; 600 species (1) 16,000
+    // 3,569 / 7,599.
+    if (n < 1 || !GroupVariantApplies(s, n))
+      return false;
+    const int64_t cells = GroupCellsPerSm(s);
+    if (n > std::min<int64_t>((int64_t)s.sm_count * (cells >= 16 ? 1024 : 820), 16384 * cells))
       return false;
     if (n == 1 && !st.gx_fn)
     {

@@ -255,6 +255,12 @@ namespace micmb
   void EnsureWorkspace(micmb_state& st, DeviceMemory& ws, int64_t doubles);
   bool GroupFaster(const micmb_solver& s, int64_t n_cells);  // than the one-cell-per-thread kernel
   bool GroupFasterThanStages(const micmb_solver& s, int64_t n_cells);  // than the plain per-stage kernels
+  // than a launch of one thread per cell, which takes about the same time for any count
+  // that the GPU holds at once, and the same again for each further set of that many;
+  // equal: the cells that a cell-group launch does in the time of one set
+  bool GroupBeatsThreads(const micmb_solver& s, int64_t n_cells, int64_t equal, const void* kernel, int block);
+  // factors of fewer entries: blocks of single warps, a few operations per launch
+  constexpr int32_t kTinyNonZeros = 128;
   void SolveFusedGroup(micmb_solver& s, micmb_state& st, const FusedArgs& A, double dt);
   // one stage of every cell (the single-stage entry points); false: not taken
   enum class GroupStage
@@ -264,7 +270,8 @@ namespace micmb
     kLu,
     kSolve
   };
-  bool LaunchGroupStage(micmb_solver& s, micmb_state& st, GroupStage stage);
+  // thread_kernel, block: the one-cell-per-thread form of it
+  bool LaunchGroupStage(micmb_solver& s, micmb_state& st, GroupStage stage, const void* thread_kernel, int block);
   // the plain method on them: per cell, or one step size for all cells; false: not taken
   bool SolvePlainPerCellGroup(micmb_solver& s, micmb_state& st, double dt, micmb_solver_stats* stats,
                               int32_t* per_cell_status, int32_t* per_cell_accepted, double* cell_time = nullptr);

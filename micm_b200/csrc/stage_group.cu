@@ -139,10 +139,36 @@ namespace micmb
     }
   }  // namespace
 
-  bool LaunchGroupStage(micmb_solver& s, micmb_state& st, GroupStage stage)
+  namespace
+  {
+    // The cells that a cell-group launch of one stage does in the time of one set of
+    // threads.  The groups bring all of a cell's arrays into shared memory and back, the
+    // threads read what a stage needs: the solve, which reads the factor once either
+    // way, has the lowest line, the LU, which reads it once per term, the highest.
+    // Measured, thousands of cells (thread kernels' time of one set: 60 species 0.29,
+    // 0.64, 0.62, 0.25 ms; TS1 1.4, 3.2, 4.1, 1.1; 600 species 3.1, 9.3, 29, 4.2):
+    //                                forcing  Jacobian   LU   solve
+    //   Chapman                         40        90      45    45
+    //   60 species (32 cells per SM)   115       125     140    62
+    //   TS1 (8)                        100       115     130    40
+    //   210 species (8)                 74        98     132    42
+    //   600 species (1)                 21        36      63    13
+    int64_t EqualCells(const micmb_solver& s, GroupStage stage)
+    {
+      static constexpr int64_t many[4] = { 770, 840, 940, 420 }, some[4] = { 500, 660, 880, 270 },
+                               one[4] = { 145, 240, 430, 88 };  // cells per SM of the GPU
+      const int i = (int)stage;
+      if (s.mech->nnz < kTinyNonZeros)
+        return 300 * (int64_t)s.sm_count;
+      const int64_t cells = GroupCellsPerSm(s);
+      return s.sm_count * (cells >= 16 ? many[i] : (cells >= 4 ? some[i] : std::min(cells * one[i], some[i])));
+    }
+  }  // namespace
+
+  bool LaunchGroupStage(micmb_solver& s, micmb_state& st, GroupStage stage, const void* thread_kernel, int block)
   {
     const int64_t n = st.n_cells;
-    if (n < 1 || !GroupFaster(s, n))
+    if (n < 1 || !GroupFaster(s, n) || !GroupBeatsThreads(s, n, EqualCells(s, stage), thread_kernel, block))
       return false;
     const GroupChoice choice = ChooseGroup(s, n);
     const StageKernel kernel = stage == GroupStage::kForcing    ? StageKernelFor<GroupStage::kForcing>(choice.G)

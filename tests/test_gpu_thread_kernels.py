@@ -7,6 +7,7 @@ from micm_b200 import Solver, micm_bench, synthetic
 from micm_b200 import solver as sv
 from micm_b200._native import check, lib
 from micm_b200.mechanism import padded_cells
+from gpu_helpers import download_cols, make_state
 from gpu_helpers import make_state
 
 pytestmark = pytest.mark.gpu
@@ -28,3 +29,79 @@ def test_alpha_minus_jacobian(cuda_device, name, n, L):
     real = (np.arange(npad) < n).reshape(-1, 1, L)
     expected += np.where(real & diagonal[None, :, None], 0.25, 0.0)
     np.testing.assert_array_equal(st.download(sv.BUF_JACOBIAN, npad * nnz), expected.ravel())
+
+
+def _inputs(n, equal=False):
+    few = micm_bench.inputs("chapman", 1000, seed=4)
+    pick = np.zeros(n, np.int64) if equal else np.arange(n) % 1000
+    return {k: np.ascontiguousarray(v[pick]) for k, v in few.items()}
+
+
+# Chapman on a GPU of 148 SMs: 44,400 cells are the last for which every stage runs on
+# cell groups, 94,720 Backward Euler; 160,000 are one set of 151,552 threads and a part
+# of the next; all of 310,000 run one cell per thread
+@pytest.mark.parametrize("n", [44400, 44401, 160000, 310000])
+def test_single_stages_on_both_sides_of_the_hand_over(cuda_device, n):
+    mech = micm_bench.mechanism("chapman")
+    inp = _inputs(n)
+    S = mech.n_species
+
+    def stages(cells):
+        solver = Solver(mech, 3, vector_length=128)
+        nnz = solver.compiled.info["jacobian_nnz"]
+        st = make_state(solver, {k: np.ascontiguousarray(v[cells]) for k, v in inp.items()})
+        solver.update_state_parameters(st)
+        out = []
+        for call, buf, cols in (("add_forcing_terms", sv.BUF_FORCING, S),
+                                ("subtract_jacobian_terms", sv.BUF_JACOBIAN, nnz),
+                                ("alpha_minus_jacobian", sv.BUF_JACOBIAN, nnz),
+                                ("lu_decompose", sv.BUF_JACOBIAN, nnz), ("linear_solve", sv.BUF_FORCING, S)):
+            args = (solver.handle, st.handle) + ((0.25,) if call == "alpha_minus_jacobian" else ())
+            check(getattr(lib(), "micmb_" + call)(*args))
+            out.append(download_cols(st, buf, cols))
+        return out
+
+    for a, b in zip(stages(slice(0, n)), stages(slice(n - 1000, n))):
+        np.testing.assert_array_equal(a[n - 1000:], b)
+
+
+@pytest.mark.parametrize("n", [94720, 94721, 160000, 310000])
+@pytest.mark.parametrize("control", ["per_cell", "global"])
+def test_backward_euler_on_both_sides_of_the_hand_over(cuda_device, n, control):
+    """Globally, a state of equal cells: the step sequence is then each cell's own."""
+    mech = micm_bench.mechanism("chapman")
+    inp = _inputs(n, equal=control == "global")
+
+    def solve(cells):
+        solver = Solver(mech, 3, vector_length=128)
+        st = make_state(solver, {k: np.ascontiguousarray(v[cells]) for k, v in inp.items()})
+        solver.update_state_parameters(st)
+        res = solver.solve_backward_euler(1000.0, st, step_control=control, per_cell=True)
+        st.sync_outputs_to_host()
+        return st.concentrations(), res
+
+    (y, r), (y_few, r_few) = solve(slice(0, n)), solve(slice(n - 1000, n))
+    np.testing.assert_array_equal(y[n - 1000:], y_few)
+    np.testing.assert_array_equal(r.per_cell_status[n - 1000:], r_few.per_cell_status)
+    np.testing.assert_array_equal(r.per_cell_accepted[n - 1000:], r_few.per_cell_accepted)
+    if control == "global":
+        assert {k: r.stats[k] for k in r.stats if k != "cells_not_converged"} == \
+            {k: r_few.stats[k] for k in r_few.stats if k != "cells_not_converged"}
+
+
+@pytest.mark.parametrize("n", [222000, 222001, 310000])
+def test_fused_on_both_sides_of_the_hand_over(cuda_device, n):
+    mech = micm_bench.mechanism("chapman")
+    inp = _inputs(n)
+
+    def solve(cells, variant):
+        solver = Solver(mech, 3, vector_length=128)
+        solver.set_fused_config(variant=variant, lu_in_shared=0)
+        st = make_state(solver, {k: np.ascontiguousarray(v[cells]) for k, v in inp.items()})
+        solver.update_state_parameters(st)
+        solver.solve(micm_bench.DT, st, method="fused", step_control="per_cell")
+        st.sync_outputs_to_host()
+        return st.concentrations()
+
+    y, y_few = solve(slice(0, n), 2), solve(slice(n - 1000, n), 0)
+    np.testing.assert_array_equal(y[n - 1000:], y_few)
