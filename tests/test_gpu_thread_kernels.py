@@ -105,3 +105,38 @@ def test_fused_on_both_sides_of_the_hand_over(cuda_device, n):
 
     y, y_few = solve(slice(0, n), 2), solve(slice(n - 1000, n), 0)
     np.testing.assert_array_equal(y[n - 1000:], y_few)
+
+
+# MICMB_BLOCKED_SCHEDULES=1: no cell groups; the same sums one cell per thread
+@pytest.mark.parametrize("name,n,L", [("c60_adjoint", 1201, 32), ("c210", 299, 128)])
+def test_stages_and_backward_euler_equal_the_cell_groups(cuda_device, monkeypatch, name, n, L):
+    """Also of cells that are not finite, statuses and counters included."""
+    mech = synthetic.CONFIGS[name]["mech"]()
+    inp = synthetic.cell_inputs(mech, n, 6, t_range=(200.0, 310.0), night_fraction=0.5)
+    inp["concentrations"][[0, 7, n - 1], 3] = np.nan, np.inf, -1.0e-9
+    got = []
+    for blocked in (True, False):
+        if blocked:
+            monkeypatch.setenv("MICMB_BLOCKED_SCHEDULES", "1")
+        else:
+            monkeypatch.delenv("MICMB_BLOCKED_SCHEDULES", raising=False)
+        solver = Solver(mech, 4, vector_length=L)
+        S, nnz = mech.n_species, solver.compiled.info["jacobian_nnz"]
+        st = make_state(solver, inp)
+        solver.update_state_parameters(st)
+        out = []
+        for call, buf, cols in (("add_forcing_terms", sv.BUF_FORCING, S),
+                                ("subtract_jacobian_terms", sv.BUF_JACOBIAN, nnz),
+                                ("alpha_minus_jacobian", sv.BUF_JACOBIAN, nnz),
+                                ("lu_decompose", sv.BUF_JACOBIAN, nnz), ("linear_solve", sv.BUF_FORCING, S)):
+            args = (solver.handle, st.handle) + ((0.25,) if call == "alpha_minus_jacobian" else ())
+            check(getattr(lib(), "micmb_" + call)(*args))
+            out.append(download_cols(st, buf, cols))
+        for control in ("per_cell", "global"):
+            st.sync_inputs_to_device()
+            res = solver.solve_backward_euler(600.0, st, step_control=control, per_cell=True)
+            st.sync_outputs_to_host()
+            out += [st.concentrations(), res.per_cell_status, res.per_cell_accepted, np.array(list(res.stats.values()))]
+        got.append(out)
+    for a, b in zip(*got):
+        np.testing.assert_array_equal(b, a)
