@@ -302,7 +302,7 @@ def flops_per_solve_unit(mech, solver, stages):
 
 def bytes_per_solve_unit(mech, solver, stages):
     """Compulsory HBM bytes of one unit of each kind of work when every working
-    set lives in HBM (the plain kernels and the one-cell-per-thread kernel):
+    set lives in HBM (the per-stage kernels and the one-cell-per-thread kernel):
     -J assembly writes the factor (zeroed, then read-modify-written), the LU
     reads and writes it, each stage solve reads it once and its vector twice,
     a forcing evaluation reads the rate constants and three state-sized
@@ -586,7 +586,9 @@ def main():
     h2d = h_vars.nbytes + h_cond.nbytes + h_par.nbytes
     d2h = h_out.nbytes
 
-    # plain per-stage kernels on the same shard (one warm-up, one timed solve)
+    # the plain method on the same shard (one warm-up, one timed solve): cell groups where
+    # an SM holds eight cells or more, one kernel per stage otherwise.  No HBM figure: on
+    # cell groups the working sets stay on chip.
     plain = None
     if args.plain_cells:
         pc = min(args.plain_cells, args.cells)
@@ -608,15 +610,10 @@ def main():
         torch.cuda.synchronize()
         pt = time.perf_counter() - t0
         (pt,) = max_over_ranks([pt], dist, "cuda")
-        plain_gbs = solve_bytes(bytes_per_solve_unit(mech, solver, cfg["stages"]), pres.stats) / pt / 1e9
         plain = {"value": pc * world / pt, "unit": UNIT, "cells_per_gpu": pc, "ms_per_step": 1000 * pt,
                  "attempts_per_cell": pres.stats["number_of_steps"] / pc,
-                 "fused_over_plain": value / (pc * world / pt),
-                 "roofline": {"bound": "hbm", "achieved": plain_gbs, "peak": peak_gbs, "unit": "GB/s",
-                              "frac": plain_gbs / peak_gbs,
-                              "note": "algorithmic bytes of the per-stage kernels over the solve's wall time "
-                                      "(launches and host synchronisation included)"}}
-        # the same kernels with micm's CUDA-path semantics: one step size for
+                 "fused_over_plain": value / (pc * world / pt)}
+        # the plain method with micm's CUDA-path semantics: one step size for
         # all cells from the error norm over all cells (a different step
         # sequence, so not bit-comparable with the per-cell solves); under
         # torchrun the step size is the whole job's: one 8-byte all-gather of

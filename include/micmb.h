@@ -341,7 +341,8 @@ int micmb_autotune(micmb_solver* solver, micmb_state* state, double dt, const ch
                    micmb_fused_config* chosen);
 
 /* CUDA-graph replay of repeated Solve calls with the fused method: captures
- * UpdateStateParameters + Solve once per (state, dt) and replays it. */
+ * UpdateStateParameters + Solve once per state, dt, tolerance, parameters and
+ * configuration, and replays it. */
 int micmb_solve_graph(micmb_solver* solver, micmb_state* state, double dt, int32_t n_repeats);
 
 /* Discrete adjoint of the accepted Rosenbrock steps of one per-cell solve
@@ -445,8 +446,8 @@ int micmb_backward_euler_params_default(micmb_backward_euler_params* out);
  * step_control MICMB_STEP_GLOBAL follows micm's multi-cell State exactly: one
  * step size and one convergence test over all cells (device-side control, one
  * launch group per Newton iteration).  MICMB_STEP_PER_CELL solves each cell as
- * micm solves a 1-cell State (one persistent kernel, one cell per thread,
- * cells taken from an atomic queue).  stats are summed over cells (global:
+ * micm solves a 1-cell State (one persistent kernel on cell groups, or one
+ * cell per thread for large counts; cells taken from an atomic queue).  stats are summed over cells (global:
  * the single control's); per_cell_status / per_cell_accepted as micmb_solve. */
 int micmb_solve_backward_euler(micmb_solver* solver, micmb_state* state, double dt,
                                const micmb_backward_euler_params* params, int32_t step_control,

@@ -12,14 +12,16 @@
 // accepted attempts in a row double H.
 //
 // Two forms:
-//   * per cell (k_backward_euler_thread): one persistent kernel, one cell per
-//     thread, each cell solved as micm solves a 1-cell State; a warp runs its
-//     cells' Newton iterations in lockstep and a thread whose cell finishes
-//     takes the next cell from an atomic counter.  Working sets live in global
-//     memory, warp-interleaved (entry e of lane l at e * 32 + l).
-//   * global (k_be_iterate / k_be_control / k_be_apply): micm's multi-cell
-//     State, one step size and one convergence test for all cells.  One
-//     thread per cell does the Newton iteration; a one-thread control kernel
+//   * per cell: one persistent kernel, each cell solved as micm solves a 1-cell
+//     State; a cell that finishes is replaced by the next from an atomic
+//     counter.  On cell groups (k_group_euler), or for large counts one cell
+//     per thread (k_backward_euler_thread): a warp runs its cells' Newton
+//     iterations in lockstep, working sets in global memory, warp-interleaved
+//     (entry e of lane l at e * 32 + l).
+//   * global (k_group_be_iterate or k_be_iterate, k_be_control, k_be_apply):
+//     micm's multi-cell State, one step size and one convergence test for all
+//     cells.  A cell group or a thread per cell does the Newton iteration; a
+//     one-thread control kernel
 //     takes micm's decisions on the device, so the host only checks for the
 //     end of the solve between batches of iterations.  The convergence test is
 //     a logical AND over all cells and species, so the result is independent

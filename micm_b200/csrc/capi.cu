@@ -1060,9 +1060,9 @@ extern "C"
         st.adj_y0 = DeviceMemory(var_bytes);
         st.adj_ybar = DeviceMemory(var_bytes);
       }
-      // The forward pass (streamed or thread variant) stores each accepted
-      // step's stage vectors beside the checkpoint, so the backward sweep (one
-      // cell per thread) rebuilds only the LU factor.
+      // The forward pass (any kernel but the direct one) stores each accepted
+      // step's stage vectors beside the checkpoint, so the backward sweep (cell
+      // groups, or one cell per thread) rebuilds only the LU factor.
       const micmb_fused_config tuned = solver->fused;
       // the direct kernel keeps no stage vectors; it also runs when variant 0 is
       // configured but the mechanism has no streamed schedule: use the thread variant
