@@ -974,7 +974,7 @@ extern "C"
       if (method == MICMB_METHOD_FUSED)
       {
         Need(step_control == MICMB_STEP_PER_CELL, "the fused method solves each cell independently (per-cell step control)");
-        SolveFused(*solver, *state, dt, stats, per_cell_status, per_cell_accepted, nullptr);
+        SolveFused(*solver, *state, dt, stats, per_cell_status, per_cell_accepted, nullptr, solver->fused);
       }
       else
         SolvePlain(*solver, *state, dt, step_control, stats, per_cell_status, per_cell_accepted);
@@ -1063,17 +1063,11 @@ extern "C"
       // The forward pass (any kernel but the direct one) stores each accepted
       // step's stage vectors beside the checkpoint, so the backward sweep (cell
       // groups, or one cell per thread) rebuilds only the LU factor.
-      const micmb_fused_config tuned = solver->fused;
+      micmb_fused_config forward = solver->fused;
       // the direct kernel keeps no stage vectors; it also runs when variant 0 is
       // configured but the mechanism has no streamed schedule: use the thread variant
-      if (tuned.variant == 1 || (tuned.variant == 0 && !StreamVariantApplies(*solver)))
-        solver->fused = micmb_fused_config{ 0, 0, 0, 0, 2 };
-      struct Restore
-      {
-        micmb_solver* s;
-        micmb_fused_config c;
-        ~Restore() { s->fused = c; }
-      } restore{ solver, tuned };
+      if (forward.variant == 1 || (forward.variant == 0 && !StreamVariantApplies(*solver, forward)))
+        forward = micmb_fused_config{ 0, 0, 0, 0, 2 };
       if (!st.adj_kbar_cells.p || st.adj_kbar_cells.bytes < sizeof(double) * (size_t)std::max<int64_t>(n * m.R, 1))
       {
         st.adj_kbar_cells = DeviceMemory(sizeof(double) * (size_t)std::max<int64_t>(n * m.R, 1));
@@ -1084,7 +1078,7 @@ extern "C"
       if (!st.accepted.p)
         st.accepted = DeviceMemory(sizeof(int32_t) * std::max<int64_t>(n, 1));
       // per-thread working sets do not shrink with the chunk: size them first
-      const int64_t ws = std::max(FusedThreadWorkspaceDoubles(*solver, n), AdjointThreadWorkspaceDoubles(*solver, n));
+      const int64_t ws = std::max(FusedThreadWorkspaceDoubles(*solver, n, forward), AdjointThreadWorkspaceDoubles(*solver, n));
       EnsureWorkspace(st, st.thread_ws, ws);
 
       // Checkpoints take max_checkpoints * (S + 1) doubles per cell, the stored
@@ -1111,7 +1105,7 @@ extern "C"
         const int64_t parts = (n + most - 1) / most;
         return std::min<int64_t>(n, ((n + parts - 1) / parts + L - 1) / L * L);
       };
-      const int64_t busy = std::min<int64_t>(n, FusedThreadResidentCells(*solver));
+      const int64_t busy = std::min<int64_t>(n, FusedThreadResidentCells(*solver, forward));
       int64_t chunk = balanced_chunk(per_cell_y + per_cell_k);
       bool store_k = true;
       if (chunk < busy && balanced_chunk(per_cell_y) > chunk)
@@ -1156,7 +1150,7 @@ extern "C"
         adj.ckpt_k = store_k ? st.adj_ckpt_k.as<double>() : nullptr;
         adj.max_ckpt = max_checkpoints;
         micmb_solver_stats cs{};
-        SolveFused(*solver, st, dt, stats ? &cs : nullptr, nullptr, nullptr, &adj);
+        SolveFused(*solver, st, dt, stats ? &cs : nullptr, nullptr, nullptr, &adj, forward);
         LaunchAdjoint(*solver, st, max_checkpoints, begin, count);
         if (stats)
         {

@@ -78,7 +78,7 @@ namespace micmb
     void EnqueueStep(micmb_solver& s, micmb_state& st, double dt)
     {
       LaunchRateConstants(s, st);
-      SolveFused(s, st, dt, nullptr, nullptr, nullptr, nullptr);
+      SolveFused(s, st, dt, nullptr, nullptr, nullptr, nullptr, s.fused);
     }
 
     void CheckFusedError(micmb_state& st)
@@ -146,11 +146,9 @@ extern "C"
       cudaEvent_t e0, e1;
       MICMB_CUDA(cudaEventCreate(&e0));
       MICMB_CUDA(cudaEventCreate(&e1));
-      const micmb_fused_config before = solver->fused;
       const bool verbose = std::getenv("MICMB_AUTOTUNE_VERBOSE") != nullptr;
       // cells per second of one configuration over the first `cells` cells (best of `reps`)
       auto rate_of = [&](const micmb_fused_config& c, int64_t cells, int reps) {
-        solver->fused = c;
         st.solve_limit = cells;
         float ms_min = -1.0f;
         for (int rep = 0; rep < reps; ++rep)
@@ -158,7 +156,7 @@ extern "C"
           MICMB_CUDA(cudaMemcpyAsync(st.variables.p, saved.p, st.variables.bytes, cudaMemcpyDeviceToDevice,
                                      st.stream));
           MICMB_CUDA(cudaEventRecord(e0, st.stream));
-          SolveFused(*solver, st, dt, nullptr, nullptr, nullptr, nullptr);
+          SolveFused(*solver, st, dt, nullptr, nullptr, nullptr, nullptr, c);
           MICMB_CUDA(cudaEventRecord(e1, st.stream));
           CheckFusedError(st);
           float ms = 0.0f;
@@ -219,7 +217,6 @@ extern "C"
       catch (...)
       {
         st.solve_limit = 0;
-        solver->fused = before;
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         throw;

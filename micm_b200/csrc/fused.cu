@@ -370,7 +370,7 @@ namespace micmb
   }  // namespace
 
   void SolveFused(micmb_solver& s, micmb_state& st, double dt, micmb_solver_stats* stats, int32_t* per_cell_status,
-                  int32_t* per_cell_accepted, const FusedArgs* adj)
+                  int32_t* per_cell_accepted, const FusedArgs* adj, const micmb_fused_config& config)
   {
     const auto& m = *s.mech;
     // an adjoint chunk brings its own cell range (n_cells > 0, pointers already offset)
@@ -379,10 +379,10 @@ namespace micmb
                           : (st.solve_limit > 0 ? std::min<int64_t>(st.solve_limit, st.n_cells) : st.n_cells);
     // variant 0 with a setting of the streamed kernel asks for that one; variant 2 without
     // a chosen build: the thread kernel where it is the faster one
-    const bool asks_streamed = s.fused.cells_per_cta > 0 || s.fused.ctas_per_sm > 0 || s.fused.ring_slots > 0;
-    const bool group = n > 0 && ((s.fused.variant == 0 && !(asks_streamed && StreamVariantApplies(s)) &&
+    const bool asks_streamed = config.cells_per_cta > 0 || config.ctas_per_sm > 0 || config.ring_slots > 0;
+    const bool group = n > 0 && ((config.variant == 0 && !(asks_streamed && StreamVariantApplies(s, config)) &&
                                   GroupVariantApplies(s, n)) ||
-                                 (s.fused.variant == 2 && s.fused.ctas_per_sm == 0 && GroupFaster(s, n)));
+                                 (config.variant == 2 && config.ctas_per_sm == 0 && GroupFaster(s, n)));
     if (group)
     {
       const FusedArgs A = PerCellArgs(st, adj, n);
@@ -390,7 +390,7 @@ namespace micmb
       ReadPerCellResults(st, A, dt, stats, per_cell_status, per_cell_accepted);
       return;
     }
-    micmb_fused_config cfg = s.fused;
+    micmb_fused_config cfg = config;
     if (cfg.lu_in_shared && FusedWarpsPerCta(s, cfg) < 1)
       cfg.lu_in_shared = 0;
     const int warps = FusedWarpsPerCta(s, cfg);
@@ -427,16 +427,16 @@ namespace micmb
       // algebraic constraints: the one-cell-per-thread kernel is the fused form that has them
       if (adj)
         throw Error(MICMB_ERR_UNSUPPORTED, "the adjoint does not cover algebraic constraints");
-      if (!SolveFusedThread(s, st, A, dt))
+      if (!SolveFusedThread(s, st, A, dt, config))
         throw Error(MICMB_ERR_UNSUPPORTED, "one-cell-per-thread kernel cannot be resident");
     }
     else if (n > 0)
     {
       bool done = false;
-      if (s.fused.variant == 0)
-        done = SolveFusedStream(s, st, dt, A);
-      else if (s.fused.variant == 2)
-        done = SolveFusedThread(s, st, A, dt);
+      if (config.variant == 0)
+        done = SolveFusedStream(s, st, dt, A, config);
+      else if (config.variant == 2)
+        done = SolveFusedThread(s, st, A, dt, config);
       if (!done)
       {
         if (A.ckpt_k)

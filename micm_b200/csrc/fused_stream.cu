@@ -514,22 +514,23 @@ namespace micmb
     return 0;
   }
 
-  bool StreamVariantApplies(const micmb_solver& s)
+  bool StreamVariantApplies(const micmb_solver& s, const micmb_fused_config& cfg)
   {
     if (!s.dev.has_warp || !s.stream_blocks.p)
       return false;
-    const int slots = std::max(2, std::min(kMaxSlots, s.fused.ring_slots > 0 ? s.fused.ring_slots : 4));
-    return StreamWarpsPerCta(s, slots, s.fused.cells_per_cta, s.fused.lu_in_shared != 0) >= 1;
+    const int slots = std::max(2, std::min(kMaxSlots, cfg.ring_slots > 0 ? cfg.ring_slots : 4));
+    return StreamWarpsPerCta(s, slots, cfg.cells_per_cta, cfg.lu_in_shared != 0) >= 1;
   }
 
-  bool SolveFusedStream(micmb_solver& s, micmb_state& st, double dt, const FusedArgs& A_in)
+  bool SolveFusedStream(micmb_solver& s, micmb_state& st, double dt, const FusedArgs& A_in,
+                        const micmb_fused_config& cfg)
   {
     const auto& m = *s.mech;
-    if (!StreamVariantApplies(s))
+    if (!StreamVariantApplies(s, cfg))
       return false;
-    const int slots = std::max(2, std::min(kMaxSlots, s.fused.ring_slots > 0 ? s.fused.ring_slots : 4));
-    const bool lu_shared = s.fused.lu_in_shared != 0;
-    const int W = StreamWarpsPerCta(s, slots, s.fused.cells_per_cta, lu_shared);
+    const int slots = std::max(2, std::min(kMaxSlots, cfg.ring_slots > 0 ? cfg.ring_slots : 4));
+    const bool lu_shared = cfg.lu_in_shared != 0;
+    const int W = StreamWarpsPerCta(s, slots, cfg.cells_per_cta, lu_shared);
     const Layout LY =
         MakeLayout(m.S, m.R, s.params.stages, (int32_t)m.info_rxn.size(), m.nnz, s.n_stream_coef, W, slots, lu_shared);
     // per-attempt block order: F0 forcing, -J, LU, then per stage [forcing], forward, backward
@@ -573,7 +574,7 @@ namespace micmb
     SA.error_flag = reinterpret_cast<int32_t*>(st.counters.as<char>() + 16);
     SA.coef = s.stream_coef.as<const double>();
     SA.n_coef = s.n_stream_coef;
-    int64_t grid = (int64_t)s.sm_count * (s.fused.ctas_per_sm > 0 ? s.fused.ctas_per_sm : 1);
+    int64_t grid = (int64_t)s.sm_count * (cfg.ctas_per_sm > 0 ? cfg.ctas_per_sm : 1);
     grid = std::max<int64_t>(1, std::min<int64_t>(grid, (A_in.n_cells + W - 1) / W));
     FusedArgs A = A_in;
     if (!lu_shared)

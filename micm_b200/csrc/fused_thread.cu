@@ -374,43 +374,44 @@ namespace micmb
       return k_fused_thread_r96<DAE>;
     }
 
-    ThreadKernel ThreadKernelFor(const micmb_solver& s)
+    ThreadKernel ThreadKernelFor(const micmb_solver& s, const micmb_fused_config& cfg)
     {
-      return s.mech->constraints.empty() ? ThreadKernelBuild<false>(s.fused) : ThreadKernelBuild<true>(s.fused);
+      return s.mech->constraints.empty() ? ThreadKernelBuild<false>(cfg) : ThreadKernelBuild<true>(cfg);
     }
 
-    int ThreadBlocksPerSm(const micmb_solver& s)
+    int ThreadBlocksPerSm(const micmb_solver& s, const micmb_fused_config& cfg)
     {
       int per_sm = 0;
-      MICMB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ThreadKernelFor(s), kThreadsPerBlock, 0));
-      if (s.fused.variant == 2 && s.fused.ctas_per_sm > 0)
-        per_sm = std::min(per_sm, s.fused.ctas_per_sm);
+      MICMB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ThreadKernelFor(s, cfg), kThreadsPerBlock, 0));
+      if (cfg.variant == 2 && cfg.ctas_per_sm > 0)
+        per_sm = std::min(per_sm, cfg.ctas_per_sm);
       return per_sm;
     }
   }  // namespace
 
-  int64_t FusedThreadResidentCells(const micmb_solver& s)
+  int64_t FusedThreadResidentCells(const micmb_solver& s, const micmb_fused_config& cfg)
   {
-    return (int64_t)std::max(ThreadBlocksPerSm(s), 1) * s.sm_count * kThreadsPerBlock;
+    return (int64_t)std::max(ThreadBlocksPerSm(s, cfg), 1) * s.sm_count * kThreadsPerBlock;
   }
 
-  int64_t FusedThreadWorkspaceDoubles(const micmb_solver& s, int64_t n_cells)
+  int64_t FusedThreadWorkspaceDoubles(const micmb_solver& s, int64_t n_cells, const micmb_fused_config& cfg)
   {
     const auto& m = *s.mech;
     const ThreadLayout T = MakeThreadLayout(m.S, m.R, s.params.stages, (int32_t)m.info_rxn.size(), m.nnz,
                                             (int32_t)m.c_term_col.size(), m.n_eq);
-    const int64_t threads = std::min<int64_t>(FusedThreadResidentCells(s),
+    const int64_t threads = std::min<int64_t>(FusedThreadResidentCells(s, cfg),
                                               (n_cells + kThreadsPerBlock - 1) / kThreadsPerBlock * kThreadsPerBlock);
     return std::max<int64_t>(threads, kThreadsPerBlock) * (int64_t)T.per_slot;
   }
 
-  bool SolveFusedThread(micmb_solver& s, micmb_state& st, const FusedArgs& A_in, double dt)
+  bool SolveFusedThread(micmb_solver& s, micmb_state& st, const FusedArgs& A_in, double dt,
+                        const micmb_fused_config& cfg)
   {
     const auto& m = *s.mech;
     const ThreadLayout T = MakeThreadLayout(m.S, m.R, s.params.stages, (int32_t)m.info_rxn.size(), m.nnz,
                                             (int32_t)m.c_term_col.size(), m.n_eq);
-    const ThreadKernel kernel = ThreadKernelFor(s);
-    const int per_sm = ThreadBlocksPerSm(s);
+    const ThreadKernel kernel = ThreadKernelFor(s, cfg);
+    const int per_sm = ThreadBlocksPerSm(s, cfg);
     if (per_sm < 1)
       return false;
     int64_t grid = (int64_t)per_sm * s.sm_count;

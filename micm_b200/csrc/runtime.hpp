@@ -219,8 +219,9 @@ namespace micmb
   // plain path: one kernel per stage; returns after the whole solve
   void SolvePlain(micmb_solver& s, micmb_state& st, double dt, int32_t step_control, micmb_solver_stats* stats,
                   int32_t* per_cell_status, int32_t* per_cell_accepted);
+  // cfg: the solver's own, or one that a call runs in its place (solvers may be shared by threads)
   void SolveFused(micmb_solver& s, micmb_state& st, double dt, micmb_solver_stats* stats, int32_t* per_cell_status,
-                  int32_t* per_cell_accepted, const FusedArgs* adjoint_ckpt);
+                  int32_t* per_cell_accepted, const FusedArgs* adjoint_ckpt, const micmb_fused_config& cfg);
   void LaunchRateConstants(micmb_solver& s, micmb_state& st);
   // single-stage launchers (per-kernel parity entry points)
   void LaunchAddForcing(micmb_solver& s, micmb_state& st);
@@ -235,11 +236,13 @@ namespace micmb
   void AllowSharedMemory(const micmb_solver& s, const void* kernel);
   size_t FusedSharedBytes(const micmb_solver& s, bool lu_in_shared);
   // streamed warp-specialised variant; returns false when it does not apply
-  bool SolveFusedStream(micmb_solver& s, micmb_state& st, double dt, const FusedArgs& A);
+  bool SolveFusedStream(micmb_solver& s, micmb_state& st, double dt, const FusedArgs& A,
+                        const micmb_fused_config& cfg);
   // whether the streamed variant runs for the solver's mechanism and configuration
-  bool StreamVariantApplies(const micmb_solver& s);
+  bool StreamVariantApplies(const micmb_solver& s, const micmb_fused_config& cfg);
   // one cell per thread, working sets in global memory
-  bool SolveFusedThread(micmb_solver& s, micmb_state& st, const FusedArgs& A, double dt);
+  bool SolveFusedThread(micmb_solver& s, micmb_state& st, const FusedArgs& A, double dt,
+                        const micmb_fused_config& cfg);
   // cell-group kernels: the block shape for n_cells cells, its work lists on the
   // device, dynamic shared memory, resident blocks (0: the cells do not fit)
   GroupChoice ChooseGroup(const micmb_solver& s, int64_t n_cells, int32_t sweep_stages = 0);
@@ -286,9 +289,9 @@ namespace micmb
   // doubles of per-thread working set the backward sweep needs for n_cells cells
   int64_t AdjointThreadWorkspaceDoubles(const micmb_solver& s, int64_t n_cells);
   // doubles of per-thread working set the one-cell-per-thread forward needs
-  int64_t FusedThreadWorkspaceDoubles(const micmb_solver& s, int64_t n_cells);
+  int64_t FusedThreadWorkspaceDoubles(const micmb_solver& s, int64_t n_cells, const micmb_fused_config& cfg);
   // cells the one-cell-per-thread forward keeps resident at once
-  int64_t FusedThreadResidentCells(const micmb_solver& s);
+  int64_t FusedThreadResidentCells(const micmb_solver& s, const micmb_fused_config& cfg);
   int FusedWarpsPerCta(const micmb_solver& s, const micmb_fused_config& cfg);
   // Backward Euler (global: micm's multi-cell State; per cell: one persistent kernel)
   void DefaultBackwardEulerParams(micmb_backward_euler_params* p);

@@ -57,3 +57,44 @@ def test_two_mechanisms_on_two_threads_equal_one_after_the_other(cuda_device, wh
     for t in threads:
         t.join(timeout=300)
     assert not errors, errors
+
+
+def test_adjoints_on_two_threads_leave_the_solver_as_it_is(cuda_device):
+    """The direct kernel keeps no stage vectors, so the adjoint's forward pass runs
+    another configuration than the solver's: that stays what it is, also seen from
+    other threads."""
+    cfg = synthetic.CONFIGS["c60_adjoint"]
+    mech = cfg["mech"]()
+    solver = Solver(mech, cfg["stages"], vector_length=32)
+    solver.set_fused_config(variant=1)
+    before = solver.get_fused_config()
+    inp = synthetic.cell_inputs(mech, 64, 5)
+    ybar = np.ones((64, mech.n_species))
+    got, seen, errors = [], [], []
+    start = threading.Barrier(2, timeout=60)
+
+    def run():
+        try:
+            import torch
+            torch.cuda.set_device(0)
+            start.wait()
+            for _ in range(10):
+                st = make_state(solver, inp)
+                solver.update_state_parameters(st)
+                g0, gk, _ = solver.solve_adjoint(600.0, st, ybar, max_checkpoints=300)
+                got.append((g0, gk))
+                seen.append(solver.get_fused_config())
+        except Exception as e:  # reported below
+            errors.append(e)
+
+    threads = [threading.Thread(target=run) for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(timeout=300)
+    assert not errors, errors
+    assert solver.get_fused_config() == before
+    assert all(c == before for c in seen)
+    for g0, gk in got[1:]:
+        np.testing.assert_array_equal(g0, got[0][0])
+        np.testing.assert_array_equal(gk, got[0][1])
