@@ -580,7 +580,7 @@ namespace micmb
     }
 
     // Whether n cells are solved by a cell-group kernel: up to where the
-    // thread-per-cell kernels are faster.  Per cell, measured, ms: Chapman 75,000 cells
+    // thread-per-cell kernels are faster.  Measured, ms, groups / threads: Chapman 75,000 cells
     // 0.188 / 0.197, 150,000 0.288 / 0.256; 60 species 303,000 36 / 147; TS1 150,000 548 /
     // 771; 210 species 262,000 197 / 767; 600 species 32,000 357 / 4,050.
     bool GroupFits(const micmb_solver& s, const void* kernel, const GroupChoice& choice, int64_t n)
